@@ -71,6 +71,7 @@ struct edus_ctx {
   double2 *d_pdiag = nullptr, *d_xw = nullptr;
   CoulDev cd{};
   void* d_part = nullptr;
+  double2* d_uev = nullptr;  // eigenvectors of the renormalised H at an output instant (8, 16 bands)
   unsigned int* d_done = nullptr;
   int* d_err = nullptr;  // device error word set by bounded waits
   edus_obs* d_log = nullptr;
@@ -302,9 +303,9 @@ int observe(edus_ctx* c) {
   // velocity gauge: the populations in the eigenbasis of H(k + A) and J1 from
   // the stencil gradient of H(k + A), as with a renormalised H
   const double2* hr = c->vg ? c->vga.H : (c->coul ? c->d_hr : nullptr);
-  CK(launch_observables(c->tb, c->d_cst, c->d_P0, hr, c->P.p.current, c->P.p.tabs, c->d_part, c->d_done, scaleJ, scaleTA,
+  CK(launch_observables(c->tb, c->d_cst, c->d_P0, hr, c->d_uev, c->P.p.current, c->P.p.tabs, c->d_part, c->d_done, scaleJ, scaleTA,
                         rec, slot, c->d_ncond, c->d_pcmax, c->stream));
-  c->launches += 1;
+  c->launches += hr && c->d_uev ? 2 : 1;
   c->nlog++;
   return 0;
 }
@@ -630,7 +631,7 @@ int dyn_enqueue_chunk(edus_ctx* c, int K, bool every) {
       const double scaleTA = std::fabs(c->P.jac) * c->P.dk[0] * c->P.dk[1] * c->P.dk[2];
       edus_obs rec;
       memset(&rec, 0, sizeof(rec));
-      CK(launch_observables(c->tb, c->d_cst, c->d_P0, c->coul ? c->d_hr : nullptr, c->P.p.current, c->P.p.tabs, c->d_part,
+      CK(launch_observables(c->tb, c->d_cst, c->d_P0, c->coul ? c->d_hr : nullptr, c->d_uev, c->P.p.current, c->P.p.tabs, c->d_part,
                             c->d_done, scaleJ, scaleTA, rec, c->d_log, c->d_ncond, c->d_pcmax, c->stream, d));
       c->launches++;
       if (c->snap_on && c->d_snap) {
@@ -1002,6 +1003,7 @@ int64_t ctx_footprint_estimate(const Problem& P) {
   double b = plane * (1 + 3 + 3 + 4 + 1 + order) + 16.0 * n * n * nk + 4.0 * P.nnb * nk;
   b += (double)(P.nprint + 2) * sizeof(edus_obs) + (double)obs_parts(P.nk) * obs_part_bytes();
   if (P.p.coulomb) {
+    b += 16.0 * (double)obs_eig_count(P.ncv, P.nk);
     const double nc = P.ncut, side = std::max(P.n1, P.n2);
     b += plane * 2 + 16.0 * 4 * nc * nc * n * n * 3 + 16.0 * 4 * nc * side * nt * 2 + 8.0 * 4 * nc * side;
   }
@@ -1556,6 +1558,7 @@ int edus_create(const edus_problem* pb, const edus_options* opt, edus_ctx** out)
       (rc = dalloc(c, &c->d_ncond, 1)) || (rc = dalloc(c, &c->d_pcmax, 1)) || (rc = dalloc(c, &c->d_maxdp, 1)) ||
       (rc = dalloc(c, &c->d_err, 1)))
     return bail(rc);
+  if ((c->coul || P.p.velocity_gauge) && obs_eig_count(n, nk) && (rc = dalloc(c, &c->d_uev, obs_eig_count(n, nk)))) return bail(rc);
   cudaMemsetAsync(c->d_ncond, 0, sizeof(double), c->stream);
   cudaMemsetAsync(c->d_done, 0, sizeof(unsigned int), c->stream);
   cudaMemsetAsync(c->d_err, 0, sizeof(int), c->stream);
@@ -2013,7 +2016,7 @@ int edus_observables(edus_ctx* c, edus_obs* out) {
   edus_obs* tmp = c->d_obs_one;
   double scaleJ = c->P.dk[0] * c->P.dk[1] * c->P.dk[2] / c->P.det_a;
   double scaleTA = std::fabs(c->P.jac) * c->P.dk[0] * c->P.dk[1] * c->P.dk[2];
-  CK(launch_observables(c->tb, c->d_cst, c->d_P0, c->vg ? c->vga.H : (c->coul ? c->d_hr : nullptr), c->P.p.current, c->P.p.tabs, c->d_part,
+  CK(launch_observables(c->tb, c->d_cst, c->d_P0, c->vg ? c->vga.H : (c->coul ? c->d_hr : nullptr), c->d_uev, c->P.p.current, c->P.p.tabs, c->d_part,
                         c->d_done, scaleJ, scaleTA, rec, tmp, nullptr, nullptr, c->stream));
   CK(cudaMemcpyAsync(out, tmp, sizeof(edus_obs), cudaMemcpyDeviceToHost, c->stream));
   CK(cudaStreamSynchronize(c->stream));
@@ -2207,7 +2210,7 @@ extern "C" int edus_observables_static(edus_ctx* c, edus_obs* out) {
   rec.dt = c->dt;
   double scaleJ = c->P.dk[0] * c->P.dk[1] * c->P.dk[2] / c->P.det_a;
   double scaleTA = std::fabs(c->P.jac) * c->P.dk[0] * c->P.dk[1] * c->P.dk[2];
-  CK(launch_observables(c->tb, c->d_cst, c->d_P0, c->vg ? c->vga.H : (c->coul ? c->d_hr : nullptr), c->P.p.current, c->P.p.tabs, base, done,
+  CK(launch_observables(c->tb, c->d_cst, c->d_P0, c->vg ? c->vga.H : (c->coul ? c->d_hr : nullptr), c->d_uev, c->P.p.current, c->P.p.tabs, base, done,
                         scaleJ, scaleTA, rec, rec_dev, nullptr, nullptr, c->stream));
   CK(cudaMemcpyAsync(out, rec_dev, sizeof(edus_obs), cudaMemcpyDeviceToHost, c->stream));
   CK(cudaStreamSynchronize(c->stream));

@@ -1,4 +1,4 @@
-// fp64.cu — Coulomb transform and observable kernels (FP64, sm_100a).
+// fp64.cu — Coulomb transform, snapshot and seam-level update kernels (FP64, sm_100a).
 //
 // k_coul_rows    first pass of the separable truncated Fourier transform of rho
 //                over the k grid (headers/Coulomb.h:300-350 restated as two 1-D
@@ -7,10 +7,6 @@
 //                shared memory and every thread owns whole dot products.
 // k_coul_modes   second pass + combination with A,B,C,D (Coulomb.h:424-466) and
 //                the first pass of the inverse transform (Coulomb.h:510-541).
-// k_obs          populations (Observables_MPI.h:217-484), J1/J2 (:668-775) and the
-//                transient absorption (:559-598) per k; the last block to finish
-//                reduces the per-block partials in a fixed order and writes the
-//                output record (no second launch, no host round trip).
 #include <cstdio>
 
 #include "dev.cuh"
@@ -188,247 +184,6 @@ __global__ void __launch_bounds__(kModeThreads) k_coul_modes(const double2* __re
     }
     h[((size_t)i1 * 2 * ncut + cs * ncut + n) * ntri + e] = cmk(ax, ay);
   }
-}
-
-// ----------------------------------------------------------------------- observables
-
-struct ObsPart {
-  double pop[kMaxBands];
-  double2 J1[3], J2[3], TA[3], PL[3];
-  double pmax, pmin;
-};
-
-__device__ __forceinline__ void obs_zero(ObsPart& p) {
-  for (int i = 0; i < kMaxBands; i++) p.pop[i] = 0;
-  for (int x = 0; x < 3; x++) p.J1[x] = p.J2[x] = p.TA[x] = p.PL[x] = cz();
-  p.pmax = 0;
-  p.pmin = 1.0;
-}
-__device__ __forceinline__ void obs_add(ObsPart& d, const ObsPart& o, int n) {
-  for (int i = 0; i < n; i++) d.pop[i] += o.pop[i];
-  for (int x = 0; x < 3; x++) {
-    d.J1[x] = cadd(d.J1[x], o.J1[x]);
-    d.J2[x] = cadd(d.J2[x], o.J2[x]);
-    d.TA[x] = cadd(d.TA[x], o.TA[x]);
-    d.PL[x] = cadd(d.PL[x], o.PL[x]);
-  }
-  d.pmax = fmax(d.pmax, o.pmax);
-  d.pmin = fmin(d.pmin, o.pmin);
-}
-
-struct ObsArgs {
-  const double2* rho;
-  const double2* hr;
-  int want_current, want_tabs;
-  ObsPart* part;
-  unsigned int* done;
-  double scaleJ, scaleTA;
-  ObsRecord rec;
-  ObsRecord* log;
-  double* ncond_dev;
-  double* pcmax_dev;
-  // adaptive step on the device: the instant is taken only when dyn->obs_now,
-  // with the clock, field and step of *dyn, into record dyn->nlog of log
-  const DynStep* dyn;
-};
-
-constexpr int kObsThreads = 128;
-
-template <int N>
-__global__ void __launch_bounds__(kObsThreads) k_obs(DevTables tb, const DevConsts* __restrict__ cst, ObsArgs a) {
-  constexpr int NT = Tri<N>::NT;
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  const int nk = tb.nk;
-  __shared__ ObsPart sp[kObsThreads];
-  __shared__ bool last;
-  ObsPart my;
-  obs_zero(my);
-  const double2* rho = a.rho;
-  const double2* hr = a.hr;
-  pdl_wait();
-  if (a.dyn && !a.dyn->obs_now) return;  // uniform: no instant at this step
-  if (k < nk) {
-    double2 P[NT];
-#pragma unroll
-    for (int e = 0; e < NT; e++) P[e] = rho[(size_t)e * nk + k];
-    auto Pf = [&](int i, int j) -> double2 { return (i <= j) ? P[Tri<N>::idx(i, j)] : cconj(P[Tri<N>::idx(j, i)]); };
-    double2 Ue[N * N];
-    if (hr) {
-      double2 A[N * N], Z[N * N];
-#pragma unroll
-      for (int i = 0; i < N; i++)
-#pragma unroll
-        for (int j = i; j < N; j++) {
-          const double2 v = hr[(size_t)Tri<N>::idx(i, j) * nk + k];
-          A[i * N + j] = v;
-          A[j * N + i] = cconj(v);
-        }
-      eig_herm_dev<N>(A, Z);
-#pragma unroll
-      for (int i = 0; i < N; i++)
-#pragma unroll
-        for (int j = 0; j < N; j++) Ue[i * N + j] = cconj(Z[j * N + i]);
-    } else {
-#pragma unroll
-      for (int e = 0; e < N * N; e++) Ue[e] = tb.U[(size_t)e * nk + k];
-    }
-#pragma unroll
-    for (int c = 0; c < N; c++) {
-      double2 acc = cz();
-#pragma unroll
-      for (int ii = 0; ii < N; ii++) {
-        double2 m = cz();
-#pragma unroll
-        for (int jj = 0; jj < N; jj++) m = cadd(m, cmul(Pf(ii, jj), Ue[c * N + jj]));
-        acc = cadd(acc, cmul(cconj(Ue[c * N + ii]), m));
-      }
-      const double Pik = acc.x;
-      my.pop[c] = Pik;
-      if (c < tb.nbands) {
-        my.pmax = fmax(my.pmax, fabs(1. - Pik));
-        my.pmin = fmin(my.pmin, 1. - Pik);
-      } else {
-        my.pmax = fmax(my.pmax, fabs(Pik));
-        my.pmin = fmin(my.pmin, Pik);
-      }
-    }
-    if (a.want_current) {
-#pragma unroll
-      for (int i = 0; i < N; i++)
-#pragma unroll
-        for (int j = i; j < N; j++) {
-          const int e = Tri<N>::idx(i, j);
-          double2 ge[3];
-          if (hr) {
-            ge[0] = ge[1] = ge[2] = cz();
-            const double2 h0 = hr[(size_t)e * nk + k];
-            for (int b = 0; b < tb.nnb; b++) {
-              const int kb = tb.nbr[(size_t)b * nk + k];
-              const double2 d = csub(hr[(size_t)e * nk + kb], h0);
-#pragma unroll
-              for (int x = 0; x < 3; x++) ge[x] = cadd(ge[x], cscale(d, cst->wb[b] * cst->bvec[b][x]));
-            }
-          } else {
-#pragma unroll
-            for (int x = 0; x < 3; x++) ge[x] = tb.GE[(size_t)(x * NT + e) * nk + k];
-          }
-#pragma unroll
-          for (int x = 0; x < 3; x++) {
-            my.J1[x] = cadd(my.J1[x], cmul(P[e], ge[x]));
-            if (i != j) my.J1[x] = cadd(my.J1[x], cmul(cconj(P[e]), cconj(ge[x])));
-          }
-        }
-      const double2* Hs = hr ? hr : tb.H;
-#pragma unroll
-      for (int i = 0; i < N; i++)
-#pragma unroll
-        for (int j = 0; j < N; j++) {
-          const double2 pij = Pf(i, j);
-#pragma unroll
-          for (int l = 0; l < N; l++) {
-            const double2 hil = (i <= l) ? Hs[(size_t)Tri<N>::idx(i, l) * nk + k] : cconj(Hs[(size_t)Tri<N>::idx(l, i) * nk + k]);
-            const double2 ph = cmul(pij, hil);
-            const int lo = j < l ? j : l, hi = j < l ? l : j;
-            // D_jl: the stored upper entry, conjugated below the diagonal for Hermitian dipoles
-            const bool cj = tb.herm_dip && j > l;
-#pragma unroll
-            for (int x = 0; x < 3; x++) {
-              const double2 ds = tb.D[(size_t)(x * NT + Tri<N>::idx(lo, hi)) * nk + k];
-              const double2 d = cj ? cconj(ds) : ds;
-              my.J2[x] = cadd(my.J2[x], cmulc(ph, d));
-            }
-          }
-        }
-    }
-    // polarisation: Tr(D_x rho) = sum_ij D_x,ij P_ij in the reference's P[k][i][j] = rho_ji
-    // convention (lower D entries: D_ji = D_ij, or conj(D_ij) for Hermitian dipoles)
-#pragma unroll
-    for (int i = 0; i < N; i++)
-#pragma unroll
-      for (int j = 0; j < N; j++) {
-        const int lo = i < j ? i : j, hi = i < j ? j : i;
-        const bool cj = tb.herm_dip && i > j;
-        const double2 pij = Pf(i, j);
-#pragma unroll
-        for (int x = 0; x < 3; x++) {
-          const double2 ds = tb.D[(size_t)(x * NT + Tri<N>::idx(lo, hi)) * nk + k];
-          my.PL[x] = cadd(my.PL[x], cmul(cj ? cconj(ds) : ds, pij));
-        }
-      }
-    if (a.want_tabs)
-      for (int i = 0; i < tb.nch; i++)
-        for (int j = tb.nch; j < N; j++) {
-          const int e = Tri<N>::idx(i, j);
-          for (int x = 0; x < 3; x++)
-            my.TA[x] = csub(my.TA[x], cmul(cscale(tb.D[(size_t)(x * NT + e) * nk + k], 2.), P[e]));
-        }
-  }
-  sp[threadIdx.x] = my;
-  __syncthreads();
-  for (int s = kObsThreads / 2; s > 0; s >>= 1) {
-    if (threadIdx.x < s) obs_add(sp[threadIdx.x], sp[threadIdx.x + s], N);
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) {
-    a.part[blockIdx.x] = sp[0];
-    __threadfence();
-    const unsigned int prev = atomicAdd(a.done, 1u);
-    last = (prev == gridDim.x - 1);
-  }
-  __syncthreads();
-  if (!last) return;
-  // last block: fixed-order reduction of all block partials
-  __threadfence();
-  ObsPart t;
-  obs_zero(t);
-  for (int b = threadIdx.x; b < gridDim.x; b += kObsThreads) obs_add(t, a.part[b], N);
-  sp[threadIdx.x] = t;
-  __syncthreads();
-  for (int s = kObsThreads / 2; s > 0; s >>= 1) {
-    if (threadIdx.x < s) obs_add(sp[threadIdx.x], sp[threadIdx.x + s], N);
-    __syncthreads();
-  }
-  if (threadIdx.x != 0) return;
-  const ObsPart& T = sp[0];
-  ObsRecord rec = a.rec;
-  ObsRecord* slot = a.log;
-  if (a.dyn) {
-    const DynStep* d = a.dyn;
-    rec.t = d->t;
-    rec.dt = d->dt;
-    for (int x = 0; x < 3; x++) {
-      rec.EF_pump[x] = d->EF_last[0][x];
-      rec.EF_probe[x] = d->EF_last[1][x];
-    }
-    slot = (a.log && d->nlog < d->log_cap) ? a.log + d->nlog : nullptr;
-  }
-  const double inv = 1. / nk;
-  double trace = -(double)tb.nbands;
-  double nc = 0;
-  for (int i = 0; i < N; i++) {
-    double v = T.pop[i] * inv;
-    trace += v;
-    if (i < tb.nbands) v = 1.0 - v;
-    rec.pop[i] = v;
-    if (v > nc) nc = v;
-  }
-  for (int x = 0; x < 3; x++) {
-    rec.J1[2 * x] = T.J1[x].x * a.scaleJ;
-    rec.J1[2 * x + 1] = T.J1[x].y * a.scaleJ;
-    rec.J2[x] = -2. * (T.J2[x].y * a.scaleJ);
-    rec.tabs[2 * x] = T.TA[x].x * a.scaleTA * inv;
-    rec.tabs[2 * x + 1] = T.TA[x].y * a.scaleTA * inv;
-    rec.pol[2 * x] = T.PL[x].x * inv;
-    rec.pol[2 * x + 1] = T.PL[x].y * inv;
-  }
-  rec.trace_dev = trace;
-  rec.p_cond_max = T.pmax;
-  rec.p_min = T.pmin;
-  rec.n_cond = nc;
-  if (slot) *slot = rec;
-  if (a.ncond_dev) *a.ncond_dev = nc;
-  if (a.pcmax_dev) *a.pcmax_dev = T.pmax;
-  *a.done = 0u;
 }
 
 // ----------------------------------------------------------------------- launchers
@@ -681,44 +436,6 @@ cudaError_t launch_axpy(const double2* a, const double2* v, double dt, double2* 
   const size_t blocks = std::min<size_t>((n + 255) / 256, 148 * 8);
   k_axpy<<<(unsigned)(blocks ? blocks : 1), 256, 0, s>>>(a, v, dt, d, n);
   return cudaGetLastError();
-}
-
-int obs_parts(int nk) { return (nk + kObsThreads - 1) / kObsThreads; }
-size_t obs_part_bytes() { return sizeof(ObsPart); }
-
-template <int N>
-static cudaError_t launch_obs_n(const DevTables& tb, const DevConsts* cst, const ObsArgs& a, cudaStream_t s) {
-  return launch_pdl(k_obs<N>, dim3(obs_parts(tb.nk)), dim3(kObsThreads), 0, s, tb, cst, a);
-}
-
-cudaError_t launch_observables(const DevTables& tb, const DevConsts* cst, const double2* rho, const double2* hr,
-                               int want_current, int want_tabs, void* part, unsigned int* done, double scaleJ,
-                               double scaleTA, const ObsRecord& rec, ObsRecord* log, double* ncond_dev,
-                               double* pcmax_dev, cudaStream_t s, const DynStep* dyn) {
-  ObsArgs a;
-  a.dyn = dyn;
-  a.rho = rho;
-  a.hr = hr;
-  a.want_current = want_current;
-  a.want_tabs = want_tabs && tb.nch > 0;
-  a.part = (ObsPart*)part;
-  a.done = done;
-  a.scaleJ = scaleJ;
-  a.scaleTA = scaleTA;
-  a.rec = rec;
-  a.log = log;
-  a.ncond_dev = ncond_dev;
-  a.pcmax_dev = pcmax_dev;
-  switch (tb.n) {
-    case 1: return launch_obs_n<1>(tb, cst, a, s);
-    case 2: return launch_obs_n<2>(tb, cst, a, s);
-    case 3: return launch_obs_n<3>(tb, cst, a, s);
-    case 4: return launch_obs_n<4>(tb, cst, a, s);
-    case 5: return launch_obs_n<5>(tb, cst, a, s);
-    case 8: return launch_obs_n<8>(tb, cst, a, s);
-    case 16: return launch_obs_n<16>(tb, cst, a, s);
-    default: return cudaErrorInvalidValue;
-  }
 }
 
 }  // namespace edus

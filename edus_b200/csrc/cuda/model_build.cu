@@ -93,6 +93,66 @@ __global__ void __launch_bounds__(64) k_wan_eig(ModelBuildArgs a) {
     }
 }
 
+// The same with N lanes per k point (8 and 16 bands, eig.cuh). Bound by the
+// chain of Jacobi rotations (28 / 120 a sweep, each a hypot, atan2 and sincos
+// and three dependent passes through shared memory), so what counts is matrices
+// in flight. A thread per k point took 7.6 ms per 16-band instance of
+// 48 x 48 to 72 x 72 and 359 us per 96 x 96 8-band instance; this form 1.17 ms and 245 us.
+constexpr int kEigThreads = 128;
+
+template <int N>
+__global__ void __launch_bounds__(kEigThreads) k_wan_eig_group(ModelBuildArgs a) {
+  constexpr int LD = EigGroup<N>::LD, M = kEigThreads / N;  // matrices per block
+  extern __shared__ double2 sm[];
+  const int m = threadIdx.x / N, r = threadIdx.x % N;
+  const int nk = a.nk, k0 = blockIdx.x * M;
+  double2* A = sm + m * EigGroup<N>::WORDS;
+  double2* Z = A + N * LD;
+  auto up = [](int i, int j) { return i * N - (i * (i - 1)) / 2 + (j - i); };
+  // upper planes, the block's k points consecutive; past the last k point the last one again
+  for (int t = threadIdx.x; t < M * N * N; t += kEigThreads) {
+    const int mk = t % M, ij = t / M, i = ij / N, j = ij % N;
+    if (i > j) continue;
+    const double2 v = a.H[(size_t)up(i, j) * nk + min(k0 + mk, nk - 1)];
+    double2* B = sm + mk * EigGroup<N>::WORDS;
+    B[i * LD + j] = v;
+    B[j * LD + i] = cconj(v);
+  }
+  __syncthreads();
+  eig_herm_group<N>(A, Z, r);
+  __syncthreads();
+  for (int t = threadIdx.x; t < M * N * N; t += kEigThreads) {
+    const int mk = t % M, ij = t / M, i = ij / N, j = ij % N, k = k0 + mk;
+    if (k >= nk) continue;
+    const double2* Zk = sm + mk * EigGroup<N>::WORDS + N * LD;
+    auto U = [&](int x, int y) { return cconj(Zk[y * LD + x]); };
+    a.U[(size_t)ij * nk + k] = U(i, j);
+    if (i > j) continue;
+    const size_t o = (size_t)up(i, j) * nk + k;
+    if (a.scissor > 1e-16) {
+      double2 v = cz();
+      for (int ii = 0; ii < N; ii++)
+        if (ii >= a.nv) v = cadd(v, cscale(cmul(cconj(U(ii, i)), U(ii, j)), a.scissor));
+      a.H[o] = cadd(a.H[o], v);
+    }
+    double2 acc = cz();
+    for (int ii = 0; ii < a.nbands; ii++) acc = cadd(acc, cmul(U(ii, i), cconj(U(ii, j))));
+    a.P0[o] = acc;
+  }
+}
+
+template <int N>
+cudaError_t launch_eig_group(const ModelBuildArgs& a, cudaStream_t s) {
+  constexpr int M = kEigThreads / N;
+  constexpr size_t smem = sizeof(double2) * EigGroup<N>::WORDS * M;
+  if (smem > 48 * 1024) {
+    cudaError_t e = cudaFuncSetAttribute(k_wan_eig_group<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+  }
+  k_wan_eig_group<N><<<(a.nk + M - 1) / M, kEigThreads, smem, s>>>(a);
+  return cudaGetLastError();
+}
+
 __global__ void k_wan_ge(ModelBuildArgs a) {
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   const int e = blockIdx.y;
@@ -146,8 +206,12 @@ cudaError_t finish_wannier_model(const ModelBuildArgs& a, cudaStream_t s) {
     case 3: k_wan_eig<3><<<blocks, 64, 0, s>>>(a); break;
     case 4: k_wan_eig<4><<<blocks, 64, 0, s>>>(a); break;
     case 5: k_wan_eig<5><<<blocks, 64, 0, s>>>(a); break;
-    case 8: k_wan_eig<8><<<blocks, 64, 0, s>>>(a); break;
-    case 16: k_wan_eig<16><<<blocks, 64, 0, s>>>(a); break;
+    case 8:
+      if ((e = launch_eig_group<8>(a, s)) != cudaSuccess) return e;
+      break;
+    case 16:
+      if ((e = launch_eig_group<16>(a, s)) != cudaSuccess) return e;
+      break;
     default: return cudaErrorInvalidValue;
   }
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
