@@ -27,6 +27,7 @@
 #include "cuda/kernels.hpp"
 #include "cuda/tc_contract.hpp"
 #include "cuda/dyn.cuh"
+#include "cuda/loop.cuh"
 #include "host/problem.hpp"
 
 namespace edus {
@@ -142,6 +143,10 @@ struct edus_ctx {
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t gexec = nullptr;
   long long graph_launches = 0;
+  // whole constant-dt runs in one launch (loop.cu): laid out once, at the first run
+  bool loop_tried = false, loop_on = false;
+  LoopArgs loop{};
+  LoopPlan loop_shape{};
   double2* d_Pinit = nullptr;
   double2 *P0_start = nullptr, *Pa_start = nullptr;
   struct HostClock {
@@ -406,13 +411,14 @@ int step_rk4(edus_ctx* c, bool startup_ring) {
   return 0;
 }
 
+const double kAbCoef[5][5] = {{1., 0, 0, 0, 0},
+                              {3.0 / 2.0, -1.0 / 2.0, 0, 0, 0},
+                              {23.0 / 12.0, -16.0 / 12.0, 5.0 / 12.0, 0, 0},
+                              {55.0 / 24.0, -59.0 / 24.0, 37.0 / 24.0, -9.0 / 24.0, 0},
+                              {1901.0 / 720.0, -2774.0 / 720.0, 2616.0 / 720.0, -1274.0 / 720.0, 251.0 / 720.0}};
+
 // Source_Main/Linear_Multistep_ODE_solvers.cpp:1-93
 int step_ab(edus_ctx* c) {
-  static const double cf[5][5] = {{1., 0, 0, 0, 0},
-                                  {3.0 / 2.0, -1.0 / 2.0, 0, 0, 0},
-                                  {23.0 / 12.0, -16.0 / 12.0, 5.0 / 12.0, 0, 0},
-                                  {55.0 / 24.0, -59.0 / 24.0, 37.0 / 24.0, -9.0 / 24.0, 0},
-                                  {1901.0 / 720.0, -2774.0 / 720.0, 2616.0 / 720.0, -1274.0 / 720.0, 251.0 / 720.0}};
   const int p = c->order;
   field_at(c->P.p, c->time_loop, c->EF);
   c->e_non0 = field_nonzero(c->EF);
@@ -431,7 +437,7 @@ int step_ab(edus_ctx* c) {
   a.dt = c->dt;
   for (int s = 0; s < p; s++) {
     a.ring_idx[s] = c->ring_idx[s];
-    a.coef[s] = cf[p - 1][s];
+    a.coef[s] = kAbCoef[p - 1][s];
   }
   a.hr_out = want_hr(c) ? c->d_hr : nullptr;
   int rc = rhs(c, a);
@@ -824,10 +830,178 @@ int run_dyn_device(edus_ctx* c) {
   return 0;
 }
 
+// ------------------------------------------------ whole run in one launch
+constexpr int kLoopChunk = 1 << 14;  // steps per launch
+
+// Plan of the run: the shape of the launch, and for every step its fields,
+// gradient coefficients and flags, along the clock of run_steps. Leaves
+// loop_on false where the run stays with the launch per stage; then the
+// context holds nothing of it.
+int loop_prepare(edus_ctx* c) {
+  c->loop_tried = true;
+  if (c->n > 5 || c->dyn || c->vg || c->coul || c->snap_on || c->solver == EDUS_SOLVER_TAYLOR || (c->solver == EDUS_SOLVER_AB && c->order > 5))
+    return 0;
+  int sms = 0, coop = 0;
+  CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device));
+  CK(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, c->device));
+  if (!coop) return 0;
+  const Problem& P = c->P;
+  const bool ab = c->solver == EDUS_SOLVER_AB;
+  const int nsteps = c->itfi + 1;
+  if (nsteps < 1) return 0;
+  std::vector<LoopStep> steps((size_t)nsteps);
+  int pmask = 0, qmask = 0;
+  {
+    double t = P.t_start, EF[2][3] = {};
+    const double dt = P.p.dt, dt2 = dt / 2.0;
+    bool non0 = true;
+    for (int it = 0; it < nsteps; it++) {
+      LoopStep& s = steps[it];
+      memset(&s, 0, sizeof(s));
+      s.t = t;
+      s.obs = it % c->res == 0;
+      memcpy(s.EF_last, EF, sizeof(EF));
+      field_at(P.p, t, EF);
+      memcpy(s.EF[0], EF, sizeof(EF));
+      if (ab) non0 = field_nonzero(EF);
+      s.e_non0 = non0;
+      s.startup = ab && P.p.ab_rk4_startup && it < c->order - 1;
+      if (!ab || s.startup) {
+        field_at(P.p, t + dt2, EF);
+        memcpy(s.EF[1], EF, sizeof(EF));
+        field_at(P.p, t + dt, EF);
+        memcpy(s.EF[2], EF, sizeof(EF));
+        non0 = field_nonzero(EF);
+      }
+      for (int q = 0; q < 3; q++)
+        for (int x = 0; x < 3; x++) {
+          if (s.EF[q][0][x] != 0.) pmask |= 1 << x;
+          if (s.EF[q][1][x] != 0.) qmask |= 1 << x;
+        }
+      t += dt;
+    }
+  }
+  // A stencil vector whose coefficients w_b E_x b_x are zero at every step adds
+  // 0 x rho: left out, unless rho can make it a NaN (models with NaN eigenvectors, kept as
+  // the reference has them)
+  bool finite = true;
+  for (const cd& v : P.P0) finite = finite && std::isfinite(v.real()) && std::isfinite(v.imag());
+  for (const cd& v : P.D) finite = finite && std::isfinite(v.real()) && std::isfinite(v.imag());
+  if (!finite) pmask = 7;
+  LoopArgs& a = c->loop;
+  int comp[3];
+  a.nb_sel = a.npc = 0;
+  for (int x = 0; x < 3; x++)
+    if ((pmask >> x) & 1) comp[a.npc++] = x;
+  for (int b = 0; b < P.nnb; b++) {
+    bool on = !finite;
+    for (int q = 0; q < a.npc; q++) on = on || (c->hc.bvec[b][comp[q]] != 0. && c->hc.wb[b] != 0.);
+    if (on) a.bsel[a.nb_sel++] = b;
+  }
+  a.nbp = std::max(12, (a.nb_sel + 5) / 6 * 6);
+  a.ngc = (3 * a.nbp * a.npc + 1) & ~1;
+  a.ncomp = 0;
+  for (int x = 0; x < 3; x++)
+    if (((pmask | qmask) >> x) & 1) a.comp[a.ncomp++] = x;
+  const LoopPlan p = loop_plan(c->tb, a.nb_sel, a.ngc, a.ncomp, sms);
+  if (p.blocks == 0) return 0;
+  a.stride = sizeof(LoopStep) + sizeof(double) * a.ngc;
+  std::vector<unsigned char> tab(a.stride * nsteps, 0);
+  for (int it = 0; it < nsteps; it++) {
+    unsigned char* row = tab.data() + a.stride * it;
+    memcpy(row, &steps[it], sizeof(LoopStep));
+    double* g = (double*)(row + sizeof(LoopStep));
+    for (int q = 0; q < 3; q++)
+      for (int s = 0; s < a.nb_sel; s++)
+        for (int u = 0; u < a.npc; u++)
+          g[(q * a.npc + u) * a.nbp + s] = c->hc.wb[a.bsel[s]] * steps[it].EF[q][0][comp[u]] * c->hc.bvec[a.bsel[s]][comp[u]];
+  }
+  unsigned char* dtab = nullptr;
+  double* dscr = nullptr;
+  unsigned int* dbar = nullptr;
+  if (dalloc(c, &dtab, tab.size()) || dalloc(c, &dscr, p.part) || dalloc(c, &dbar, 1)) {
+    clear_error();
+    cudaGetLastError();  // no memory for it: the launch per stage needs none
+    return 0;
+  }
+  CK(cudaMemcpyAsync(dtab, tab.data(), tab.size(), cudaMemcpyHostToDevice, c->stream));
+  CK(cudaStreamSynchronize(c->stream));
+  a.steps = dtab;
+  a.part = dscr;
+  a.bar = dbar;
+  a.tb = c->tb;
+  a.cst = c->d_cst;
+  a.order = ab ? c->order : 0;
+  a.res = c->res;
+  a.nstartup = ab && P.p.ab_rk4_startup ? c->order - 1 : 0;
+  a.kt = p.kt;
+  a.cluster = p.cluster;
+  a.P1 = c->d_P1;
+  a.Pb = c->d_Pb;
+  a.ring = c->d_ring;
+  a.dt = P.p.dt;
+  a.dt6 = a.dt / 6.0;
+  a.dt3 = a.dt / 3.0;
+  a.dt2 = a.dt / 2.0;
+  a.wx2 = P.p.probe.wl;
+  for (int q = 0; q < kMaxOrder; q++) a.coef[q] = ab && q < c->order ? kAbCoef[c->order - 1][q] : 0.;
+  a.want_current = P.p.current;
+  a.want_tabs = P.p.tabs && P.nch > 0;
+  a.scaleJ = P.dk[0] * P.dk[1] * P.dk[2] / P.det_a;
+  a.scaleTA = std::fabs(P.jac) * P.dk[0] * P.dk[1] * P.dk[2];
+  a.ncond_dev = c->d_ncond;
+  a.pcmax_dev = c->d_pcmax;
+  c->loop_shape = p;
+  c->loop_on = true;
+  return 0;
+}
+
+// The whole run from it = 0 as launches of up to kLoopChunk steps; the host
+// clock advances as run_steps leaves it.
+int loop_run(edus_ctx* c) {
+  c->P0_start = c->d_P0;
+  c->Pa_start = c->d_Pa;
+  LoopArgs a = c->loop;
+  while (c->it <= c->itfi) {
+    a.P0 = c->d_P0;
+    a.Pa = c->d_Pa;
+    a.steps = c->loop.steps + a.stride * c->it;
+    a.it0 = c->it;
+    a.nsteps = std::min(kLoopChunk, c->itfi + 1 - c->it);
+    a.log = c->d_log + c->nlog;
+    a.log_cap = c->log_cap - c->nlog;
+    CK(cudaMemsetAsync(a.bar, 0, sizeof(unsigned int), c->stream));
+    CK(launch_loop(a, c->loop_shape, c->stream));
+    c->launches++;
+    for (int s = 0; s < a.nsteps; s++) {
+      if (c->it % c->res == 0) c->nlog++;
+      const bool ab = c->solver == EDUS_SOLVER_AB, startup = ab && c->P.p.ab_rk4_startup && c->it < c->order - 1;
+      if (ab) {
+        const int fill = c->ring_idx[c->order - 1];
+        for (int q = c->order - 1; q > 0; q--) c->ring_idx[q] = c->ring_idx[q - 1];
+        c->ring_idx[0] = fill;
+        if (!startup) std::swap(c->d_P0, c->d_Pa);
+      }
+      c->time_loop += c->dt;
+      c->it++;
+    }
+  }
+  // the field of the last evaluation
+  double tl = c->P.t_start;
+  for (int s = 0; s + 1 < c->it; s++) tl += c->dt;
+  if (c->solver == EDUS_SOLVER_AB && !(c->P.p.ab_rk4_startup && c->itfi < c->order - 1)) {
+    field_at(c->P.p, tl, c->EF);
+  } else {
+    field_at(c->P.p, tl + c->dt, c->EF);
+  }
+  c->e_non0 = field_nonzero(c->EF);
+  return 0;
+}
+
 // Enqueue nsteps (or the whole run) between the context's two timing events;
 // *l0 receives the launch count before them. timed_finish waits for the end
 // event and checks the device error word.
-int timed_start(edus_ctx* c, int nsteps, bool all, long long* l0_out) {
+int timed_start(edus_ctx* c, int nsteps, bool all, long long* l0_out, bool alone = true) {
   CK(cudaSetDevice(c->device));
   long long l0 = c->launches;
   *l0_out = l0;
@@ -839,6 +1013,21 @@ int timed_start(edus_ctx* c, int nsteps, bool all, long long* l0_out) {
     return 0;
   }
   const bool graph = all && !c->dyn && c->use_graphs && c->it == 0;
+  // (a run that shares the GPU with a batch keeps the graph: its small kernels
+  // run beside the batch's, blocks that wait on one another would not)
+  if (graph && alone && !c->profiling) {
+    if (!c->loop_tried) {
+      int rc = loop_prepare(c);
+      if (rc) return rc;
+    }
+    if (c->loop_on) {
+      CK(cudaEventRecord(c->ev0, c->stream));
+      int rc = loop_run(c);
+      if (rc) return rc;
+      CK(cudaEventRecord(c->ev1, c->stream));
+      return 0;
+    }
+  }
   if (graph && !c->gexec) {
     // capture the whole loop once; the captured kernels run at cudaGraphLaunch below
     c->P0_start = c->d_P0;
@@ -968,7 +1157,7 @@ int ctx_start_async(edus_ctx* c) {
   if (!c) return fail(EDUS_EINVAL, "null argument");
   if (c->dyn || !c->use_graphs || c->it != 0)
     return fail(EDUS_EUNSUPPORTED, "an asynchronous whole run needs a fresh context at constant dt with graphs");
-  return timed_start(c, 0, true, &c->async_l0);
+  return timed_start(c, 0, true, &c->async_l0, false);
 }
 
 int ctx_poll(edus_ctx* c, bool* done) {

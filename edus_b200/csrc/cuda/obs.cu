@@ -18,6 +18,7 @@
 #include "dyn.cuh"
 #include "eig.cuh"
 #include "kernels.hpp"
+#include "obs.cuh"
 
 namespace edus {
 
@@ -29,15 +30,7 @@ struct Tri {
   static __device__ __forceinline__ int idx(int i, int j) { return i * N - (i * (i - 1)) / 2 + (j - i); }
 };
 
-// fields of a partial: populations, then per component x J1 re, J1 im, J2 im,
-// TA re, TA im, polarisation re, im, then max and min
-constexpr int kFX = kMaxBands;
-constexpr int kPerX = 7;
-constexpr int kFMax = kFX + 3 * kPerX, kFMin = kFMax + 1;
-constexpr int kFields = kFMin + 1;
-
 // Sums of one k point, thread or block in k_obs.
-
 struct ObsPart {
   double pop[kMaxBands];
   double2 J1[3], J2[3], TA[3], PL[3];
@@ -85,22 +78,6 @@ static_assert(kFields * sizeof(double) <= sizeof(ObsPart), "partials are sized b
 // blocks of k_obs_el: enough for three 256- or two 512-thread blocks on every SM
 constexpr int kObsElBlocks = 512;
 
-__device__ __forceinline__ double obs_op(int f, double a, double b) {
-  return f == kFMax ? fmax(a, b) : (f == kFMin ? fmin(a, b) : a + b);
-}
-
-// One warp: value f of 128 consecutive entries (four per lane) as a binary tree
-// over 128; the result is lane 0's.
-__device__ __forceinline__ double tree128(int f, double v0, double v1, double v2, double v3) {
-  double x = obs_op(f, obs_op(f, v0, v2), obs_op(f, v1, v3));
-  for (int s = 16; s > 0; s >>= 1) x = obs_op(f, x, __shfl_down_sync(0xffffffffu, x, s));
-  return x;
-}
-
-// Field v of a block that carries N populations, in the partial's numbering.
-template <int N>
-__device__ __forceinline__ int field_no(int v) { return v < N ? v : kFX + (v - N); }
-
 // The output record from the totals T of every field (one thread).
 template <int N>
 __device__ __forceinline__ void obs_record(const DevTables& tb, const ObsArgs& a, const double* T) {
@@ -116,30 +93,7 @@ __device__ __forceinline__ void obs_record(const DevTables& tb, const ObsArgs& a
     }
     slot = (a.log && d->nlog < d->log_cap) ? a.log + d->nlog : nullptr;
   }
-  const double inv = 1. / tb.nk;
-  double trace = -(double)tb.nbands;
-  double nc = 0;
-  for (int i = 0; i < N; i++) {
-    double v = T[i] * inv;
-    trace += v;
-    if (i < tb.nbands) v = 1.0 - v;
-    rec.pop[i] = v;
-    if (v > nc) nc = v;
-  }
-  for (int x = 0; x < 3; x++) {
-    const double* f = T + kFX + kPerX * x;
-    rec.J1[2 * x] = f[0] * a.scaleJ;
-    rec.J1[2 * x + 1] = f[1] * a.scaleJ;
-    rec.J2[x] = -2. * (f[2] * a.scaleJ);
-    rec.tabs[2 * x] = f[3] * a.scaleTA * inv;
-    rec.tabs[2 * x + 1] = f[4] * a.scaleTA * inv;
-    rec.pol[2 * x] = f[5] * inv;
-    rec.pol[2 * x + 1] = f[6] * inv;
-  }
-  rec.trace_dev = trace;
-  rec.p_cond_max = T[kFMax];
-  rec.p_min = T[kFMin];
-  rec.n_cond = nc;
+  const double nc = obs_fill(rec, T, N, tb.nk, tb.nbands, a.scaleJ, a.scaleTA);
   if (slot) *slot = rec;
   if (a.ncond_dev) *a.ncond_dev = nc;
   if (a.pcmax_dev) *a.pcmax_dev = T[kFMax];

@@ -1,0 +1,72 @@
+"""Whole constant-dt solves in one launch (k_loop) against the launch per stage on
+the same problem, at the sizes where the split over blocks can go wrong: a
+block that is partly filled, one cluster and many blocks, the largest grids the
+form takes and the first it leaves to the launch per stage, every band count it
+is built for, several launches in a row."""
+import numpy as np
+import pytest
+
+import edus_b200 as E
+from edus_b200 import workloads as W
+
+pytestmark = pytest.mark.gpu
+
+
+def make(workdir, kind, n1, n2, solver, res, t_fin=0.35):
+    kw = dict(n=n1, field=0.5, photon=1.6, duration=0.8, t_fin_fs=t_fin, it_res=res)
+    if kind == "hbn":
+        path = W.hbn_rk4(workdir, solver=solver, **kw)
+    else:
+        path = W.wannier(workdir, nw=kind, nside=5, name="W", pol="0 1 1", **kw)
+    text = open(path).read().replace(f"1 {n1} {n1}\n", f"1 {n1} {n2}\n")
+    with open(path, "w") as f:
+        f.write(text)
+    return E.Problem(E.parse_input(path), workdir)
+
+
+AB4 = "Adams_Bashforth 4\nAdams_Bashforth_RK4_startup\n"
+
+
+@pytest.mark.parametrize("kind,n1,n2,solver,one", [
+    ("hbn", 4, 4, "", True),       # one block of 16 k points
+    ("hbn", 30, 32, "", True),     # 960 = 15 x 64 k points: the largest cluster
+    ("hbn", 30, 34, "", True),     # the first grid past it
+    ("hbn", 60, 62, AB4, True),    # last block partly filled
+    ("hbn", 98, 98, "", True),     # more than kLoopSmall threads a block
+    ("hbn", 124, 124, "", True),   # 105 k points a block, the last that fits
+    ("hbn", 126, 126, "", False),  # launch per stage
+    (2, 12, 14, "", True),
+    (4, 12, 14, "", True),
+    (5, 20, 22, "", True),
+    (5, 80, 80, "", False),
+])
+def test_one_launch_matches_launch_per_stage(workdir, kind, n1, n2, solver, one):
+    pb = make(workdir, kind, n1, n2, solver, 3)
+    a, b = E.Context(pb), E.Context(pb, use_graphs=False)
+    for _ in range(2):  # a second run after a reset
+        a.run()
+        assert (a.last_timing()[1] == 1) == one
+        b.run()
+        # the stage arithmetic is the same expression by expression: the repository's bar for rho
+        assert np.abs(a.get_state() - b.get_state()).max() <= 1e-13
+        la, lb = a.obs(), b.obs()
+        assert len(la) == len(lb)
+        for q in ("t", "J1", "J2", "pol", "pop", "EF_pump", "trace_dev", "p_cond_max", "p_min", "n_cond", "dt"):
+            x, y = np.array([o[q] for o in la]), np.array([o[q] for o in lb])
+            # k sums in another order: FP64 rounding of sums whose terms are at most a few a.u.
+            assert np.abs(x - y).max() <= 1e-12, q
+        assert a.clock() == b.clock()
+        a.reset()
+        b.reset()
+
+
+def test_run_of_several_launches_keeps_the_history(workdir):
+    """More steps than one launch takes: Adams-Bashforth's derivatives cross the gap."""
+    pb = make(workdir, "hbn", 8, 8, "Adams_Bashforth 5\n", 500, t_fin=170.0)
+    assert pb.info.nsteps > 1 << 14
+    a, b = E.Context(pb), E.Context(pb, use_graphs=False)
+    a.run()
+    assert a.last_timing()[1] == 2
+    b.run()
+    assert np.abs(a.get_state() - b.get_state()).max() <= 1e-13
+    assert len(a.obs()) == len(b.obs())
