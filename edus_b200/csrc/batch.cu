@@ -373,33 +373,25 @@ int build_model_tc(edus_batch* b, const Problem& P, const Inst& I) {
   // H and D on the tensor cores; dH/dk, an observable-only table whose k sums
   // cancel strongly, is the reference's stencil over an FP64 H(k) (CUDA cores)
   const int ncomp = 4;
-  const int kp = tc_pad_k(nr), kseg = tc_seg_k(nr), ncols = 2 * ncomp * nt, K = 2 * nr;
-  std::vector<uint16_t> Bw((size_t)ncols * kp, 0);
-  std::vector<double> col(K);
+  const int kp = tc_pad_k(nr), ncols = 2 * ncomp * nt;
+  // upper coefficients of H(R) and the symmetrised dipoles; the scale of a GEMM
+  // column is the power of two that brings every value into [-1/2, 1/2)
+  std::vector<double2> coef((size_t)ncomp * nt * nr);
+  std::vector<double> colscale(ncols);
   for (int i = 0; i < n; i++)
     for (int j = i; j < n; j++) {
       const int e = tri_index(i, j, n);
       for (int comp = 0; comp < ncomp; comp++) {
         const int ce = comp * nt + e;
-        for (int part = 0; part < 2; part++) {
-          // re column: [Re c ; -Im c], im column: [Im c ; Re c]
-          double amax = 0.;
-          for (int r = 0; r < nr; r++) {
-            const cd c = comp == 0 ? P.HR[((size_t)i * n + j) * nr + r]
-                                   : 0.5 * (P.rR[(((size_t)(comp - 1) * n + i) * n + j) * nr + r] +
-                                            P.rR[(((size_t)(comp - 1) * n + j) * n + i) * nr + r]);
-            col[r] = part == 0 ? c.real() : c.imag();
-            col[nr + r] = part == 0 ? -c.imag() : c.real();
-            amax = std::max(amax, std::max(std::fabs(col[r]), std::fabs(col[nr + r])));
-          }
-          // power-of-two scale of the column: every y = value / scale in [-1/2, 1/2), so every
-          // slice is at most 128 in magnitude; the phases enter halved, so the stored
-          // slices carry 2 scale
-          const double scale = amax > 0. ? std::ldexp(1.0, std::ilogb(amax) + 2) : 1.0;
-          uint16_t* row = &Bw[(size_t)(2 * ce + part) * kp];
-          for (int p = 0; p < kTcPairs; p++)
-            for (int q = 0; q < K; q++) row[(size_t)p * kseg + q] = tc_bf16(2.0 * scale * tc_slice(col[q] / scale, tc_pair_b(p)));
+        double amax = 0.;
+        for (int r = 0; r < nr; r++) {
+          const cd c = comp == 0 ? P.HR[((size_t)i * n + j) * nr + r]
+                                 : 0.5 * (P.rR[(((size_t)(comp - 1) * n + i) * n + j) * nr + r] +
+                                          P.rR[(((size_t)(comp - 1) * n + j) * n + i) * nr + r]);
+          coef[(size_t)ce * nr + r] = mkc<double2>(c);
+          amax = std::max(amax, std::max(std::fabs(c.real()), std::fabs(c.imag())));
         }
+        colscale[2 * ce] = colscale[2 * ce + 1] = amax > 0. ? std::ldexp(1.0, std::ilogb(amax) + 2) : 1.0;
       }
     }
   std::vector<double2> hdr((size_t)n * nr);
@@ -409,13 +401,11 @@ int build_model_tc(edus_batch* b, const Problem& P, const Inst& I) {
   for (int bb = 0; bb < P.nnb; bb++)
     for (int x = 0; x < 3; x++) gb[bb * 3 + x] = P.shell_w[P.bshell[bb]] * P.bvec[bb * 3 + x];
   const size_t plane = (size_t)nt * nk;
-  const size_t bytes = align256(sizeof(double) * 3 * nk) + align256(sizeof(double) * 3 * nr) + align256(sizeof(uint16_t) * Bw.size()) +
-                       align256(sizeof(double2) * hdr.size()) + align256(sizeof(double) * gb.size()) +
+  const size_t bytes = align256(sizeof(double) * 3 * nk) + align256(sizeof(double) * 3 * nr) + align256(sizeof(double2) * coef.size()) +
+                       align256(sizeof(double) * ncols) + align256(sizeof(uint16_t) * (size_t)ncols * kp) + align256(sizeof(double2) * hdr.size()) + align256(sizeof(double) * gb.size()) +
                        align256(sizeof(uint16_t) * (size_t)nk * kp) + align256(sizeof(double) * (size_t)nk * ncols) +
                        align256(sizeof(double2) * plane) + align256(sizeof(double2) * n * n * nk) +
-                       (I.GE ? align256(sizeof(double2) * plane) + align256(sizeof(double2) * 3 * plane) +
-                                   align256(sizeof(double2) * 4 * nt * nr)
-                             : 0);
+                       (I.GE ? align256(sizeof(double2) * plane) + align256(sizeof(double2) * 3 * plane) : 0);
   char* base = nullptr;
   if (cudaMallocAsync((void**)&base, bytes, b->pool, b->stream) != cudaSuccess) {
     cudaGetLastError();
@@ -429,11 +419,12 @@ int build_model_tc(edus_batch* b, const Problem& P, const Inst& I) {
   };
   double* dk = (double*)carve(sizeof(double) * 3 * nk);
   double* dR = (double*)carve(sizeof(double) * 3 * nr);
-  uint16_t* dB = (uint16_t*)carve(sizeof(uint16_t) * Bw.size());
+  double2* dcoef = (double2*)carve(sizeof(double2) * coef.size());
+  double* dscale = (double*)carve(sizeof(double) * ncols);
   double2* dh = (double2*)carve(sizeof(double2) * hdr.size());
   double* dg = (double*)carve(sizeof(double) * gb.size());
   int rc;
-  if ((rc = put(b, dk, P.kpt)) || (rc = put(b, dR, P.Rvec)) || (rc = put(b, dB, Bw)) || (rc = put(b, dh, hdr)) || (rc = put(b, dg, gb))) {
+  if ((rc = put(b, dk, P.kpt)) || (rc = put(b, dR, P.Rvec)) || (rc = put(b, dcoef, coef)) || (rc = put(b, dscale, colscale)) || (rc = put(b, dh, hdr)) || (rc = put(b, dg, gb))) {
     cudaFreeAsync(base, b->stream);
     return rc;
   }
@@ -444,7 +435,9 @@ int build_model_tc(edus_batch* b, const Problem& P, const Inst& I) {
   t.nr = nr;
   t.kpt = dk;
   t.Rvec = dR;
-  t.Bw = dB;
+  t.coef = dcoef;
+  t.colscale = dscale;
+  t.Bw = (uint16_t*)carve(sizeof(uint16_t) * (size_t)ncols * kp);
   t.hdiagR = dh;
   t.Aw = (uint16_t*)carve(sizeof(uint16_t) * (size_t)nk * kp);
   t.Cw = (double*)carve(sizeof(double) * (size_t)nk * ncols);
@@ -475,22 +468,12 @@ int build_model_tc(edus_batch* b, const Problem& P, const Inst& I) {
   if (e == cudaSuccess) e = finish_wannier_model(a, b->stream);
   if (e == cudaSuccess) e = planes_to_float(a.U, (float2*)I.U, (size_t)n * n * nk, b->stream);
   if (e == cudaSuccess && I.GE) {
-    // dH/dk: FP64 H(k) (coefficients: H(R) upper elements) and the stencil
-    std::vector<double2> hc((size_t)nt * nr);
-    for (int i = 0; i < n; i++)
-      for (int j = i; j < n; j++)
-        for (int r = 0; r < nr; r++) hc[(size_t)tri_index(i, j, n) * nr + r] = mkc<double2>(P.HR[((size_t)i * n + j) * nr + r]);
+    // dH/dk: FP64 H(k) (its coefficients come first) and the stencil
     ModelBuildArgs g = a;
     g.only_h = 1;
     g.H = (double2*)carve(sizeof(double2) * plane);
     g.GE = (double2*)carve(sizeof(double2) * 3 * plane);
-    double2* dhc = (double2*)carve(sizeof(double2) * 4 * nt * nr);
-    int prc = put(b, dhc, hc);
-    if (prc) {
-      cudaFreeAsync(base, b->stream);
-      return prc;
-    }
-    g.coef = dhc;
+    g.coef = dcoef;
     e = wannier_h_and_gradient(g, b->stream);
     if (e == cudaSuccess) e = planes_to_float(g.GE, (float2*)I.GE, 3 * plane, b->stream);
   }

@@ -594,10 +594,13 @@ __global__ void __launch_bounds__(kWsThreads, 2) k_tc_gemm_ws(const __grid_const
   if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(2 * kTmemCols2));
 }
 
-// Velocity gauge: coefficient slices of c_A(R) = e^{2 pi i A.R} c(R), one thread per
+// Coefficient slices of c_A(R) = e^{2 pi i A.R} c(R) (velocity gauge; the model
+// build of a batch instance has A = 0, where c_A = c exactly), one thread per
 // (column, K entry); column 2 ce + part holds [Re c_A ; -Im c_A] (part 0) or
-// [Im c_A ; Re c_A] (part 1), pre-multiplied by 2 scale as the host build's slices
-__global__ void k_vg_bslices(const double2* __restrict__ coef, const double* __restrict__ Rvec, const double* __restrict__ colscale,
+// [Im c_A ; Re c_A] (part 1), divided by the column's scale, cut and pre-multiplied
+// by 2 scale (the phases enter halved). 2.1 us for 8 bands and 121 R vectors; cut
+// on the host for every admitted instance it was 3 ms of one core.
+__global__ void k_bslices(const double2* __restrict__ coef, const double* __restrict__ Rvec, const double* __restrict__ colscale,
                              double A0, double A1, double A2, int ntri, int nr, int kseg, int kpad, uint16_t* __restrict__ B) {
   const int q = blockIdx.x * blockDim.x + threadIdx.x;  // K entry
   const int col = blockIdx.y;                          // 2 (comp * ntri + e) + part
@@ -652,6 +655,10 @@ cudaError_t tc_contract(const TcArgs& a, cudaStream_t s) {
   k_phase_split<<<a.nk, 256, 0, s>>>(a.kpt, a.Rvec, a.nk, a.nr, tc_seg_k(a.nr), kpad, a.Aw);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
+  if ((e = cudaMemsetAsync(a.Bw, 0, sizeof(uint16_t) * (size_t)ncols * kpad, s)) != cudaSuccess) return e;  // segment padding
+  k_bslices<<<dim3((2 * a.nr + 127) / 128, ncols), 128, 0, s>>>(a.coef, a.Rvec, a.colscale, 0., 0., 0., a.ntri, a.nr, tc_seg_k(a.nr),
+                                                               kpad, a.Bw);
+  if ((e = cudaGetLastError()) != cudaSuccess) return e;
   CUtensorMap mA, mB;
   const bool tma = tc_gemm_tma_wanted() && tc_gemm_maps(a.Aw, a.Bw, a.nk, ncols, kpad, &mA, &mB) == cudaSuccess;
   if ((e = tc_gemm_run(a.Aw, a.Bw, a.Cw, a.nk, ncols, kpad, tc_seg_k(a.nr), a.err, tma ? &mA : nullptr, tma ? &mB : nullptr, s)) !=
@@ -762,7 +769,7 @@ cudaError_t tc_vg_maps(TcVgArgs& a) {
 
 cudaError_t tc_vg_stage(const TcVgArgs& a, cudaStream_t s) {
   const int kpad = tc_pad_k(a.nr), kseg = tc_seg_k(a.nr), ncols = 8 * a.ntri;
-  k_vg_bslices<<<dim3((2 * a.nr + 127) / 128, ncols), 128, 0, s>>>(a.coef, a.Rvec, a.colscale, a.A[0], a.A[1], a.A[2], a.ntri,
+  k_bslices<<<dim3((2 * a.nr + 127) / 128, ncols), 128, 0, s>>>(a.coef, a.Rvec, a.colscale, a.A[0], a.A[1], a.A[2], a.ntri,
                                                                    a.nr, kseg, kpad, a.Bw);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;

@@ -14,7 +14,9 @@ struct TcArgs {
   int n, ntri, nk, nr;
   const double* kpt;     // [nk][3]
   const double* Rvec;    // [nr][3]
-  const uint16_t* Bw;    // [8 ntri][Kp] coefficient slices (BF16), one K segment per slice pair (host-built)
+  const double2* coef;   // [4][ntri][nr]: H(R), (r_x(R) + r_x(R)^T) / 2 upper entries
+  const double* colscale;  // [8 ntri] power-of-two scale of each GEMM column
+  uint16_t* Bw;          // scratch [8 ntri][Kp] coefficient slices (BF16), one K segment per slice pair
   const double2* hdiagR; // [n][nr] H_ii(R) for the FP64 band energies
   uint16_t* Aw;          // scratch [nk][Kp] phase slices (BF16), one K segment per slice pair
   double* Cw;            // scratch [nk][8 ntri] GEMM result (FP64 sum of FP32 slices)
