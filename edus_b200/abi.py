@@ -192,6 +192,22 @@ def obs_to_dict(o, ncv):
     }
 
 
+def obs_list(buf, count, ncv):
+    """The first `count` records of an Obs array as obs_to_dict gives them, read in bulk."""
+    import numpy as np
+
+    a = np.frombuffer(buf, dtype=np.dtype(Obs), count=count)
+
+    def cplx(name):
+        return np.ascontiguousarray(a[name]).view(np.complex128)
+
+    keys = ("t", "EF_pump", "EF_probe", "J1", "J2", "pop", "tabs", "trace_dev", "p_cond_max", "p_min", "n_cond", "dt", "pol")
+    cols = (a["t"].tolist(), a["EF_pump"].copy(), a["EF_probe"].copy(), cplx("J1"), a["J2"].copy(), a["pop"][:, :ncv].copy(),
+            cplx("tabs"), a["trace_dev"].tolist(), a["p_cond_max"].tolist(), a["p_min"].tolist(), a["n_cond"].tolist(),
+            a["dt"].tolist(), cplx("pol"))
+    return [dict(zip(keys, row)) for row in zip(*cols)]
+
+
 class BatchOptions(C.Structure):
     _fields_ = [
         ("device", C.c_int32),

@@ -17,6 +17,7 @@
 
 #include "ctx_hooks.hpp"
 #include "cuda/batch.cuh"
+#include "cuda/kernels.hpp"
 #include "cuda/model_build.hpp"
 #include "cuda/tc_contract.hpp"
 #include "host/problem.hpp"
@@ -30,6 +31,8 @@ namespace {
     cudaError_t e_ = (x);                                                                 \
     if (e_ != cudaSuccess) return fail(EDUS_ECUDA, "%s: %s", #x, cudaGetErrorString(e_)); \
   } while (0)
+
+constexpr size_t kStageBytes = 4 << 20;  // one pinned buffer
 
 size_t align256(size_t b) { return (b + 255) & ~(size_t)255; }
 
@@ -107,6 +110,9 @@ struct edus_batch {
   double device_ms = 0, kpoint_steps = 0;
   long long launches = 0;
   long long h2d_bytes = 0, d2h_bytes = 0;
+  // pinned buffers of copy_out, allocated by the first state that is read
+  void* stage[2] = {nullptr, nullptr};
+  cudaEvent_t stage_ev[2] = {nullptr, nullptr};
 };
 
 namespace {
@@ -144,7 +150,7 @@ Layout layout_of(const edus_batch* b, const Problem& P, int kt) {
   L.field = align256((size_t)(P.itfi + 2) * sizeof(FieldRow));
   const int res = std::max(1, P.p.it_resolution);
   L.log = align256((size_t)(P.itfi / res + 1) * sizeof(edus_obs));
-  L.part = align256(((nk + kt - 1) / kt) * obs_part_bytes());
+  L.part = align256(((nk + kt - 1) / kt) * batch::obs_part_bytes());
   return L;
 }
 
@@ -222,18 +228,6 @@ double2 mkc<double2>(const cd& v) { return make_double2(v.real(), v.imag()); }
 template <>
 float2 mkc<float2>(const cd& v) { return make_float2((float)v.real(), (float)v.imag()); }
 
-// reference layout [k][n][n](x comps) -> upper-triangle planes [x][e][k]
-template <class T>
-void planes(const cd* src, int nk, int n, int comps, std::vector<T>& dst) {
-  const int nt = n * (n + 1) / 2;
-  dst.resize((size_t)comps * nt * nk);
-  for (int k = 0; k < nk; k++)
-    for (int i = 0; i < n; i++)
-      for (int j = i; j < n; j++)
-        for (int x = 0; x < comps; x++)
-          dst[((size_t)x * nt + tri_index(i, j, n)) * nk + k] = mkc<T>(src[(((size_t)k * n + i) * n + j) * comps + x]);
-}
-
 template <class T>
 int put(edus_batch* b, void* d, const std::vector<T>& h) {
   BCK(cudaMemcpyAsync(d, h.data(), sizeof(T) * h.size(), cudaMemcpyHostToDevice, b->stream));
@@ -241,30 +235,38 @@ int put(edus_batch* b, void* d, const std::vector<T>& h) {
   return 0;
 }
 
+// A table in the reference's layout to the instance's planes: sent as it lies and
+// laid out by the device, through the scratch (room for the widest table).
+template <class T>
+int put_planes(edus_batch* b, const std::vector<cd>& src, int nk, int n, int comps, bool full, T* dst, double2* scratch) {
+  BCK(cudaMemcpyAsync(scratch, src.data(), sizeof(cd) * src.size(), cudaMemcpyHostToDevice, b->stream));
+  b->h2d_bytes += (long long)(sizeof(cd) * src.size());
+  BCK(launch_to_planes(scratch, nk, n, comps, full, dst, b->stream));
+  return 0;
+}
+
 template <class T>
 int upload_model(edus_batch* b, const Problem& P, const Inst& I) {
   const int n = P.ncv, nk = P.nk;
-  std::vector<T> pl;
-  int rc;
-  planes<T>(P.H.data(), nk, n, 1, pl);
-  if ((rc = put(b, (void*)I.H, pl))) return rc;
-  planes<T>(P.D.data(), nk, n, 3, pl);
-  if ((rc = put(b, (void*)I.D, pl))) return rc;
-  if (I.GE) {
-    planes<T>(P.GE.data(), nk, n, 3, pl);
-    if ((rc = put(b, (void*)I.GE, pl))) return rc;
+  double2* scr = nullptr;
+  if (cudaMallocAsync((void**)&scr, sizeof(double2) * 3 * n * n * nk, b->pool, b->stream) != cudaSuccess) {
+    cudaGetLastError();
+    return fail(EDUS_ENOMEM, "batch: upload scratch of %zu bytes", sizeof(double2) * 3 * n * n * nk);
   }
-  pl.resize((size_t)n * n * nk);
-  for (int k = 0; k < nk; k++)
-    for (int e = 0; e < n * n; e++) pl[(size_t)e * nk + k] = mkc<T>(P.U[(size_t)k * n * n + e]);
-  if ((rc = put(b, (void*)I.U, pl))) return rc;
-  if (I.Hdiag) {
+  int rc = put_planes(b, P.H, nk, n, 1, false, (T*)I.H, scr);
+  if (!rc) rc = put_planes(b, P.D, nk, n, 3, false, (T*)I.D, scr);
+  if (!rc && I.GE) rc = put_planes(b, P.GE, nk, n, 3, false, (T*)I.GE, scr);
+  if (!rc) rc = put_planes(b, P.U, nk, n, 1, true, (T*)I.U, scr);
+  if (!rc && I.Hdiag) {
     std::vector<double> hd((size_t)n * nk);
     for (int k = 0; k < nk; k++)
       for (int i = 0; i < n; i++) hd[(size_t)i * nk + k] = P.H[((size_t)k * n + i) * n + i].real();
-    if ((rc = put(b, (void*)I.Hdiag, hd))) return rc;
+    rc = put(b, (void*)I.Hdiag, hd);
   }
-  return 0;
+  // mixed precision: the state is the deviation from rho_eq
+  if (!rc) rc = put_planes(b, P.P0, nk, n, 1, false, I.Peq ? const_cast<double2*>(I.Peq) : I.P0, scr);
+  cudaFreeAsync(scr, b->stream);
+  return rc;
 }
 
 // Field components and stencil vectors that contribute for the whole run. A
@@ -353,15 +355,17 @@ void detect_lattice(const Problem& P, Inst& I) {
     I.off[b][0] = d1;
     I.off[b][1] = d2;
   }
-  for (int k = 0; k < P.nk; k++) {
-    const int i1 = k / n2, i2 = k % n2;
-    for (int b = 0; b < P.nnb; b++) {
-      const int j1 = ((i1 + I.off[b][0]) % n1 + n1) % n1, j2 = ((i2 + I.off[b][1]) % n2 + n2) % n2;
-      if (P.nbr[(size_t)k * P.nnb + b] != j1 * n2 + j2) return;
-    }
-  }
   for (int b = 0; b < P.nnb; b++)
     if (I.off[b][0] <= -n1 || I.off[b][0] >= n1 || I.off[b][1] <= -n2 || I.off[b][1] >= n2) return;
+  const int* nb = P.nbr.data();
+  for (int i1 = 0; i1 < n1; i1++)
+    for (int i2 = 0; i2 < n2; i2++)
+      for (int b = 0; b < P.nnb; b++) {
+        int j1 = i1 + I.off[b][0], j2 = i2 + I.off[b][1];
+        j1 += j1 < 0 ? n1 : (j1 >= n1 ? -n1 : 0);
+        j2 += j2 < 0 ? n2 : (j2 >= n2 ? -n2 : 0);
+        if (*nb++ != j1 * n2 + j2) return;
+      }
   I.lattice = 1;
 }
 
@@ -751,6 +755,42 @@ int run_chunk(edus_batch* b, LaunchTimer* tm = nullptr) {
   return 0;
 }
 
+// Device memory to the caller's (pageable) memory: two pinned buffers take turns,
+// the copy of one over PCIe running while the threads of the host empty the other.
+// The driver's own path for pageable memory fills the caller's fresh pages on one
+// thread. Waits for the stream.
+cudaError_t copy_out(edus_batch* b, void* dst, const void* src, size_t bytes) {
+  if (bytes < kStageBytes / 4) {
+    cudaError_t e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, b->stream);
+    return e == cudaSuccess ? cudaStreamSynchronize(b->stream) : e;
+  }
+  for (int q = 0; q < 2; q++) {
+    cudaError_t e = cudaSuccess;
+    if (!b->stage[q]) e = cudaHostAlloc(&b->stage[q], kStageBytes, cudaHostAllocDefault);
+    if (e == cudaSuccess && !b->stage_ev[q]) e = cudaEventCreateWithFlags(&b->stage_ev[q], cudaEventDisableTiming);
+    if (e != cudaSuccess) return e;
+  }
+  const size_t nchunk = (bytes + kStageBytes - 1) / kStageBytes;
+  auto size = [&](size_t c) { return std::min(kStageBytes, bytes - c * kStageBytes); };
+  auto start = [&](size_t c) {
+    cudaError_t e = cudaMemcpyAsync(b->stage[c & 1], (const char*)src + c * kStageBytes, size(c), cudaMemcpyDeviceToHost, b->stream);
+    return e == cudaSuccess ? cudaEventRecord(b->stage_ev[c & 1], b->stream) : e;
+  };
+  cudaError_t e = start(0);
+  for (size_t c = 0; c < nchunk && e == cudaSuccess; c++) {
+    if (c + 1 < nchunk && (e = start(c + 1)) != cudaSuccess) break;
+    if ((e = cudaEventSynchronize(b->stage_ev[c & 1])) != cudaSuccess) break;
+    char* d = (char*)dst + c * kStageBytes;
+    const char* from = (const char*)b->stage[c & 1];
+    constexpr size_t kPiece = 256 << 10;
+    const long pieces = (long)((size(c) + kPiece - 1) / kPiece);
+#pragma omp parallel for schedule(static) num_threads(8)
+    for (long q = 0; q < pieces; q++) memcpy(d + q * kPiece, from + q * kPiece, std::min(kPiece, size(c) - q * kPiece));
+  }
+  if (e != cudaSuccess) cudaStreamSynchronize(b->stream);  // nothing left in flight towards the buffers
+  return e;
+}
+
 Slot* slot_of(edus_batch* b, int32_t slot) {
   if (!b || slot < 0 || slot >= (int)b->slots.size()) return nullptr;
   return &b->slots[slot];
@@ -952,6 +992,10 @@ void edus_batch_destroy(edus_batch* b) {
   cudaFree(b->d_it[0]);
   cudaFree(b->d_it[1]);
   cudaFree(b->d_err);
+  for (int q = 0; q < 2; q++) {
+    if (b->stage[q]) cudaFreeHost(b->stage[q]);
+    if (b->stage_ev[q]) cudaEventDestroy(b->stage_ev[q]);
+  }
   if (b->pool) cudaMemPoolDestroy(b->pool);
   if (b->e0) cudaEventDestroy(b->e0);
   if (b->e1) cudaEventDestroy(b->e1);
@@ -1072,16 +1116,8 @@ int edus_batch_add(edus_batch* b, const edus_problem* pb, int64_t tag, int32_t* 
   } else {
     rc = cmix(b, n) ? upload_model<float2>(b, P, I) : upload_model<double2>(b, P, I);
     if (rc) return undo(rc);
-    std::vector<double2> st;
-    planes<double2>(P.P0.data(), nk, n, 1, st);
-    if (I.Peq) {
-      // mixed precision: the state is the deviation from rho_eq
-      if ((rc = put(b, (void*)I.Peq, st))) return undo(rc);
-      if (cudaMemsetAsync(I.P0, 0, sizeof(double2) * st.size(), b->stream) != cudaSuccess)
-        return undo(fail(EDUS_ECUDA, "batch: clear deviation"));
-    } else if ((rc = put(b, I.P0, st))) {
-      return undo(rc);
-    }
+    if (I.Peq && cudaMemsetAsync(I.P0, 0, sizeof(double2) * (size_t)nt * nk, b->stream) != cudaSuccess)
+      return undo(fail(EDUS_ECUDA, "batch: clear deviation"));
   }
   // mixed precision: Pb starts as the FP32 copy of the deviation P0 = 0 that
   // stage 0 reads (stage 3 refreshes it every step)
@@ -1203,26 +1239,19 @@ int edus_batch_get_state(edus_batch* b, int32_t slot, double* rho) {
     return rc;
   }
   BCK(cudaSetDevice(b->device));
-  const int n = s->n, nk = s->nk;
-  std::vector<double2> pl((size_t)s->ntri * nk);
-  BCK(cudaMemcpyAsync(pl.data(), s->inst.P0, sizeof(double2) * pl.size(), cudaMemcpyDeviceToHost, b->stream));
-  std::vector<double2> eq;
-  if (s->inst.Peq) {
-    // mixed precision keeps the deviation from rho_eq
-    eq.resize(pl.size());
-    BCK(cudaMemcpyAsync(eq.data(), s->inst.Peq, sizeof(double2) * eq.size(), cudaMemcpyDeviceToHost, b->stream));
+  // full matrices on the device (mixed precision keeps the deviation from
+  // rho_eq), then out through the batch's pinned buffers
+  const size_t bytes = sizeof(double2) * (size_t)s->n * s->n * s->nk;
+  double2* full = nullptr;
+  if (cudaMallocAsync((void**)&full, bytes, b->pool, b->stream) != cudaSuccess) {
+    cudaGetLastError();
+    return fail(EDUS_ENOMEM, "batch: %zu bytes for the state's matrices", bytes);
   }
-  BCK(cudaStreamSynchronize(b->stream));
-  b->d2h_bytes += (long long)(sizeof(double2) * (pl.size() + eq.size()));
-  for (size_t q = 0; q < eq.size(); q++) pl[q] = cadd(pl[q], eq[q]);
-  cd* o = (cd*)rho;
-  for (int k = 0; k < nk; k++)
-    for (int i = 0; i < n; i++)
-      for (int j = i; j < n; j++) {
-        const double2 v = pl[(size_t)tri_index(i, j, n) * nk + k];
-        o[((size_t)k * n + i) * n + j] = cd(v.x, v.y);
-        if (i != j) o[((size_t)k * n + j) * n + i] = cd(v.x, -v.y);
-      }
+  cudaError_t e = launch_from_planes(s->inst.P0, s->inst.Peq, s->nk, s->n, full, b->stream);
+  if (e == cudaSuccess) e = copy_out(b, rho, full, bytes);
+  cudaFreeAsync(full, b->stream);
+  BCK(e);
+  b->d2h_bytes += (long long)bytes;
   return 0;
 }
 

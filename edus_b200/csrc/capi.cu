@@ -147,6 +147,7 @@ struct edus_ctx {
   bool loop_tried = false, loop_on = false;
   LoopArgs loop{};
   LoopPlan loop_shape{};
+  double2* d_full = nullptr;  // matrices of state_from_dev, allocated on its first call
   double2* d_Pinit = nullptr;
   double2 *P0_start = nullptr, *Pa_start = nullptr;
   struct HostClock {
@@ -202,11 +203,24 @@ int state_to_dev(edus_ctx* c, const double* rho, double2* d) {
   return 0;
 }
 
+// Full matrices on the device, then straight to the caller; the first call takes
+// the room for them, and without it the host lays the planes out.
 int state_from_dev(edus_ctx* c, const double2* d, double* rho) {
+  const int n = c->n, nk = c->nk;
+  const size_t bytes = sizeof(double2) * (size_t)n * n * nk;
+  if (!c->d_full && dalloc(c, &c->d_full, (size_t)n * n * nk)) {
+    clear_error();
+    cudaGetLastError();
+  }
+  if (c->d_full) {
+    CK(launch_from_planes(d, nullptr, nk, n, c->d_full, c->stream));
+    CK(cudaMemcpyAsync(rho, c->d_full, bytes, cudaMemcpyDeviceToHost, c->stream));
+    CK(cudaStreamSynchronize(c->stream));
+    return 0;
+  }
   std::vector<double2> pl(c->plane);
   CK(cudaMemcpyAsync(pl.data(), d, sizeof(double2) * c->plane, cudaMemcpyDeviceToHost, c->stream));
   CK(cudaStreamSynchronize(c->stream));
-  const int n = c->n, nk = c->nk;
   cd* out = (cd*)rho;
   for (int k = 0; k < nk; k++)
     for (int i = 0; i < n; i++)

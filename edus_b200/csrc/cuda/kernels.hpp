@@ -50,6 +50,12 @@ cudaError_t launch_axpy(const double2* a, const double2* v, double dt, double2* 
 // Wannier basis from the inverse-transform rows tb.h.
 cudaError_t launch_pdiag(const DevTables& tb, const double2* rho, double2* pd, cudaStream_t s);
 cudaError_t launch_coulomb_xw(const DevTables& tb, const DevConsts* cst, const double2* pd, double2* xw, cudaStream_t s);
+// Reference layout [k][n][n](x comps) to planes [comp][e][k] of the upper triangle
+// (full: of every entry), rounded to FP32 for float2; and planes P (+ Q when not
+// null) to full Hermitian matrices [k][n][n] (layout.cu).
+cudaError_t launch_to_planes(const double2* src, int nk, int n, int comps, bool full, double2* dst, cudaStream_t s);
+cudaError_t launch_to_planes(const double2* src, int nk, int n, int comps, bool full, float2* dst, cudaStream_t s);
+cudaError_t launch_from_planes(const double2* P, const double2* Q, int nk, int n, double2* dst, cudaStream_t s);
 // Velocity gauge: H(k + A), D(k + A) of a Wannier model at every k point
 // (vgauge.cu). coef: [4][ntri][nr] upper-triangle coefficients of H(R) and of
 // the symmetric dipoles (r_x(R) + r_x(R)^T) / 2; A in crystal coordinates.

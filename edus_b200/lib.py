@@ -276,7 +276,7 @@ class Context:
         _check(self._L.edus_obs_count(self._h, C.byref(n)), "edus_obs_count")
         buf = (abi.Obs * max(n.value, 1))()
         _check(self._L.edus_obs_get(self._h, 0, n.value, buf), "edus_obs_get")
-        return [abi.obs_to_dict(buf[i], self.n) for i in range(n.value)]
+        return abi.obs_list(buf, n.value, self.n)
 
     def observables(self):
         o = abi.Obs()
@@ -407,7 +407,7 @@ class Batch:
         buf = (abi.Obs * max(n.value, 1))()
         if n.value:
             _check(self._L.edus_batch_obs_get(self._h, int(slot), 0, n.value, buf), "edus_batch_obs_get")
-        return [abi.obs_to_dict(buf[i], self._n[slot]) for i in range(n.value)]
+        return abi.obs_list(buf, n.value, self._n[slot])
 
     def get_state(self, slot):
         n, nk = self._n[slot], self._nk[slot]
@@ -508,7 +508,7 @@ class Server:
         buf = (abi.Obs * max(i["nobs"], 1))()
         if i["nobs"]:
             _check(self._L.edus_server_obs(self._h, int(rid), 0, i["nobs"], buf), "edus_server_obs")
-        return [abi.obs_to_dict(buf[q], i["nbands"]) for q in range(i["nobs"])]
+        return abi.obs_list(buf, i["nobs"], i["nbands"])
 
     def forget(self, rid):
         _check(self._L.edus_server_forget(self._h, int(rid)), "edus_server_forget")
