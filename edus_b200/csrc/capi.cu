@@ -147,6 +147,9 @@ struct edus_ctx {
   bool loop_tried = false, loop_on = false;
   LoopArgs loop{};
   LoopPlan loop_shape{};
+  // initial state and dipoles finite, and the largest stencil weight (select_terms)
+  bool finite = true;
+  double wb_max = 0;
   double2* d_full = nullptr;  // matrices of state_from_dev, allocated on its first call
   double2* d_Pinit = nullptr;
   double2 *P0_start = nullptr, *Pa_start = nullptr;
@@ -194,7 +197,26 @@ int upload(edus_ctx* c, double2* d, const std::vector<double2>& h) {
   return 0;
 }
 
+// A state from outside that is not finite: from here on no term is left out
+// (select_terms), and a plan made for fewer terms is made again.
+void note_state(edus_ctx* c, const double* rho) {
+  if (!c->finite) return;
+  const size_t count = (size_t)2 * c->n * c->n * c->nk;
+  for (size_t q = 0; q < count && c->finite; q++) c->finite = std::isfinite(rho[q]);
+  if (c->finite) return;
+  if (c->gexec) cudaGraphExecDestroy(c->gexec);
+  if (c->graph) cudaGraphDestroy(c->graph);
+  c->gexec = nullptr;
+  c->graph = nullptr;
+  if (c->dyn_exec) cudaGraphExecDestroy(c->dyn_exec);
+  if (c->dyn_graph) cudaGraphDestroy(c->dyn_graph);
+  c->dyn_exec = nullptr;
+  c->dyn_graph = nullptr;
+  c->loop_tried = c->loop_on = false;
+}
+
 int state_to_dev(edus_ctx* c, const double* rho, double2* d) {
+  note_state(c, rho);
   std::vector<double2> pl;
   to_planes((const cd*)rho, c->nk, c->n, 1, pl);
   int rc = upload(c, d, pl);
@@ -283,7 +305,39 @@ int run_coulomb(edus_ctx* c, const double2* src) {
   return prof_mark(c, 1, false);
 }
 
+// The terms of a stage that are not exact zeros. A shell weight below 1e-12 of
+// the largest is least-squares noise of the weight fit (1e-21 against 1e3 for the
+// diagonal shell of a square grid), its terms far below the FP64 resolution of the
+// sum; batches leave the same ones out. With a state or dipoles that are not
+// finite 0 x NaN counts, and nothing is left out.
+void select_terms(const edus_ctx* c, StageArgs& a) {
+  int pmask = 0, qmask = 0;
+  if (a.dyn) {
+    // the fields live on the device: every component some laser can have
+    const edus_params& p = c->P.p;
+    for (int x = 0; x < 3; x++) {
+      for (int q = 0; q < p.n_pumps; q++)
+        if (p.pump[q].pol1[x] != 0. || p.pump[q].pol2[x] != 0.) pmask |= 1 << x;
+      if (p.probe.pol1[x] != 0. || p.probe.pol2[x] != 0.) qmask |= 1 << x;
+    }
+  } else {
+    for (int x = 0; x < 3; x++) {
+      if (a.EF[0][x] != 0.) pmask |= 1 << x;
+      if (a.EF[1][x] != 0.) qmask |= 1 << x;
+    }
+  }
+  a.dmask = c->finite ? pmask | qmask : 7;
+  a.nsel = 0;
+  for (int b = 0; b < c->tb.nnb; b++) {
+    bool on = !c->finite;
+    if (std::fabs(c->hc.wb[b]) > 1e-12 * c->wb_max)
+      for (int x = 0; x < 3; x++) on = on || (((pmask >> x) & 1) && c->hc.bvec[b][x] != 0.);
+    if (on) a.sel[a.nsel++] = (unsigned char)b;
+  }
+}
+
 int rhs(edus_ctx* c, StageArgs& a) {
+  select_terms(c, a);
   int rc = run_coulomb(c, a.src);
   if (rc) return rc;
   if ((rc = prof_mark(c, 0, true))) return rc;
@@ -898,9 +952,7 @@ int loop_prepare(edus_ctx* c) {
   // A stencil vector whose coefficients w_b E_x b_x are zero at every step adds
   // 0 x rho: left out, unless rho can make it a NaN (models with NaN eigenvectors, kept as
   // the reference has them)
-  bool finite = true;
-  for (const cd& v : P.P0) finite = finite && std::isfinite(v.real()) && std::isfinite(v.imag());
-  for (const cd& v : P.D) finite = finite && std::isfinite(v.real()) && std::isfinite(v.imag());
+  const bool finite = c->finite;
   if (!finite) pmask = 7;
   LoopArgs& a = c->loop;
   int comp[3];
@@ -909,7 +961,7 @@ int loop_prepare(edus_ctx* c) {
     if ((pmask >> x) & 1) comp[a.npc++] = x;
   for (int b = 0; b < P.nnb; b++) {
     bool on = !finite;
-    for (int q = 0; q < a.npc; q++) on = on || (c->hc.bvec[b][comp[q]] != 0. && c->hc.wb[b] != 0.);
+    for (int q = 0; q < a.npc; q++) on = on || (c->hc.bvec[b][comp[q]] != 0. && std::fabs(c->hc.wb[b]) > 1e-12 * c->wb_max);
     if (on) a.bsel[a.nb_sel++] = b;
   }
   a.nbp = std::max(12, (a.nb_sel + 5) / 6 * 6);
@@ -1737,6 +1789,9 @@ int edus_create(const edus_problem* pb, const edus_options* opt, edus_ctx** out)
     h.wb[b] = P.shell_w[P.bshell[b]];
     for (int x = 0; x < 3; x++) h.bvec[b][x] = P.bvec[b * 3 + x];
   }
+  for (int b = 0; b < P.nnb; b++) c->wb_max = std::max(c->wb_max, std::fabs(h.wb[b]));
+  for (const cd& v : P.P0) c->finite = c->finite && std::isfinite(v.real()) && std::isfinite(v.imag());
+  for (const cd& v : P.D) c->finite = c->finite && std::isfinite(v.real()) && std::isfinite(v.imag());
   for (int i = 0; i < n; i++)
     for (int j = 0; j < n; j++) h.T[i * n + j] = P.T[i][j];
   for (size_t t = 0; t < P.diss_i.size(); t++) {

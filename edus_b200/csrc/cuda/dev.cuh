@@ -186,6 +186,11 @@ struct StageArgs {
   unsigned long long* maxdp;
   double pcond_plus_ncond;  // P_cond_max + n_cond
   int stage_rows;           // set by the launcher: k-grid rows of Coulomb tables staged per block
+  // terms of this stage that can be nonzero, in order (set by the caller): stencil
+  // vectors whose coefficient w_b (E_pump . b) is not identically zero, bit x of
+  // dmask for the field components in use
+  int nsel, dmask;
+  unsigned char sel[kMaxNb];
   // Coulomb in the diagonal basis: the mean-field term already rotated back to
   // the Wannier basis, [ntri][nk] (null: the Wannier-basis term from tb.h)
   const double2* xw;

@@ -11,6 +11,12 @@
 // Source_Main/Taylor_DE_solver_deriv_Polynom.cpp:142-177). Compared with a
 // thread per k this gives NT times the parallelism for the small grids of the
 // reference's workloads, where one solve has only 10^3-10^4 k points.
+//
+// Bound by L2: with 8 and 16 bands most of a stage's bytes are the stencil
+// gathers and the dipole planes. Stencil vectors orthogonal to the field (8 of 12
+// on a square grid with the field along an axis) and dipole components without a
+// field are left out: their terms are exact zeros. 96 x 96, 8 bands: 20.5 us a
+// stage, 25.2 with all of them; 30 x 34, 16 bands: 16.6, 17.6.
 #include "dev.cuh"
 #include "dyn.cuh"
 #include "kernels.hpp"
@@ -99,7 +105,8 @@ __global__ void __launch_bounds__(KT* TriEP<N>::NT) k_rhs_ep(DevTables tb, const
     Pe = a.src[(size_t)e * nk + k];
     He = tb.H[(size_t)e * nk + k];
 #pragma unroll
-    for (int x = 0; x < 3; x++) De[x] = tb.D[(size_t)(x * NT + e) * nk + k];
+    for (int x = 0; x < 3; x++)
+      if ((a.dmask >> x) & 1) De[x] = tb.D[(size_t)(x * NT + e) * nk + k];
   }
   if (staged) {
     __syncthreads();  // trig table + barrier init visible to all threads
@@ -168,7 +175,8 @@ __global__ void __launch_bounds__(KT* TriEP<N>::NT) k_rhs_ep(DevTables tb, const
     if (e_non0) {
       // sum_b (w_b E_pump . b) rho_e(k + b)
 #pragma unroll 6
-      for (int b = 0; b < tb.nnb; b++) {
+      for (int c = 0; c < a.nsel; c++) {
+        const int b = a.sel[c];
         const int kb = tb.nbr[(size_t)b * nk + k];
         const double2 pn = a.src[(size_t)e * nk + kb];
         const double f0 = cst->wb[b] * ef0[0] * cst->bvec[b][0];
