@@ -17,6 +17,11 @@
 // on a square grid with the field along an axis) and dipole components without a
 // field are left out: their terms are exact zeros. 96 x 96, 8 bands: 20.5 us a
 // stage, 25.2 with all of them; 30 x 34, 16 bands: 16.6, 17.6.
+//
+// 8 and 16 bands exchange full matrices (RowsEP): every operand of the commutator is
+// a constant offset from four row pointers, where triangles need an index, a
+// branch and a conjugation per operand. 96 x 96, 8 bands: 14.2 us a stage, 20.5 with
+// triangles; 30 x 34, 16 bands: 11.6, 16.6.
 #include "dev.cuh"
 #include "dyn.cuh"
 #include "kernels.hpp"
@@ -38,14 +43,32 @@ struct TriEP {
   }
 };
 
+// Exchange rows of the full-matrix form (8 and 16 bands): entry (r, c) of k point
+// kl at [r * RS + c * KT + kl]; the padded row stride puts the rows that the
+// elements (i, j), (i, j + 1), ... of a warp read on different banks.
+template <int N, int KT>
+struct RowsEP {
+  static constexpr bool FULL = N >= 8;
+  static constexpr int RS = N * KT + KT, SIZE = FULL ? N * RS : 1;
+  // Resident blocks the registers are sized for. 8 bands: three blocks of 288
+  // threads (8 k points; 62.3 us a step on 96 x 96), against 73.8 for two of 576 and
+  // 73.5 for four of 288, which spill, and 87.6 for one of 576 as the element-parallel
+  // form ran. 16 bands: one block of 544 (51.3 us on 30 x 34; two 53.8, three 68.6).
+  static constexpr int BLOCKS = N == 8 ? 3 : (N == 16 ? 1 : 1);
+};
+
 // DYN: the stage scalars come from the adaptive step's device copy (a.dyn);
 // a separate instantiation so the constant-step kernel keeps its registers.
 template <int N, int KT, bool DYN>
-__global__ void __launch_bounds__(KT* TriEP<N>::NT) k_rhs_ep(DevTables tb, const DevConsts* __restrict__ cst, StageArgs a) {
+__global__ void __launch_bounds__(KT* TriEP<N>::NT, RowsEP<N, KT>::BLOCKS) k_rhs_ep(DevTables tb, const DevConsts* __restrict__ cst, StageArgs a) {
   constexpr int NT = TriEP<N>::NT;
-  __shared__ double2 sP[NT][KT];
-  __shared__ double2 sHu[NT][KT];  // H~_ij, i <= j
-  __shared__ double2 sHl[NT][KT];  // H~_ji, i <= j (D is symmetric, H Hermitian)
+  using Rows = RowsEP<N, KT>;
+  constexpr bool FULL = Rows::FULL;
+  constexpr int RS = Rows::RS;
+  __shared__ double2 sP[FULL ? 1 : NT][KT];
+  __shared__ double2 sHu[FULL ? 1 : NT][KT];  // H~_ij, i <= j
+  __shared__ double2 sHl[FULL ? 1 : NT][KT];  // H~_ji, i <= j (D is symmetric, H Hermitian)
+  __shared__ double2 fP[Rows::SIZE], fH[Rows::SIZE];  // full matrices
   extern __shared__ double2 dyn[];  // Coulomb row tables: h rows [nrows][2][ncut][NT], trig [2][ncut][KT]
   const int kl = threadIdx.x, e = threadIdx.y;
   const int k0 = blockIdx.x * KT;
@@ -201,22 +224,50 @@ __global__ void __launch_bounds__(KT* TriEP<N>::NT) k_rhs_ep(DevTables tb, const
       hu = cadd(hu, cscale(De[x], f));
       hl = cadd(hl, cscale(herm ? cconj(De[x]) : De[x], f));
     }
-    sP[e][kl] = Pe;
-    sHu[e][kl] = hu;
-    sHl[e][kl] = hl;
+    if constexpr (FULL) {
+      fP[i * RS + j * KT + kl] = Pe;
+      fP[j * RS + i * KT + kl] = i == j ? Pe : cconj(Pe);
+      fH[i * RS + j * KT + kl] = hu;
+      if (i != j) fH[j * RS + i * KT + kl] = hl;
+    } else {
+      sP[e][kl] = Pe;
+      sHu[e][kl] = hu;
+      sHl[e][kl] = hl;
+    }
   }
   __syncthreads();
 
   double dpmax = 0.;
   if (valid) {
     auto Pf = [&](int r, int c) -> double2 {
+      if constexpr (FULL) return fP[r * RS + c * KT + kl];
       return (r <= c) ? sP[TriEP<N>::idx(r, c)][kl] : cconj(sP[TriEP<N>::idx(c, r)][kl]);
     };
     auto HF = [&](int r, int c) -> double2 {
       return (r <= c) ? sHu[TriEP<N>::idx(r, c)][kl] : sHl[TriEP<N>::idx(c, r)][kl];
     };
     double2 v;
-    if (i == j) {
+    if constexpr (FULL) {
+      // beta_ij = sum_l H~_jl P_il - conj(H~_il P_jl) for every element (2 i Im of one
+      // sum on the diagonal) as multiply-adds into eight partial sums
+      const double2 *Hi = fH + i * RS + kl, *Hj = fH + j * RS + kl, *Pi = fP + i * RS + kl, *Pj = fP + j * RS + kl;
+      double ax[2] = {0., 0.}, ay[2] = {0., 0.}, bx[2] = {0., 0.}, by[2] = {0., 0.};
+#pragma unroll
+      for (int l = 0; l < N; l++) {
+        const int q = l & 1;
+        const double2 hj = Hj[l * KT], pi = Pi[l * KT], hi = Hi[l * KT], pj = Pj[l * KT];
+        ax[q] = fma(hj.x, pi.x, ax[q]);
+        ax[q] = fma(-hj.y, pi.y, ax[q]);
+        ay[q] = fma(hj.x, pi.y, ay[q]);
+        ay[q] = fma(hj.y, pi.x, ay[q]);
+        bx[q] = fma(hi.x, pj.x, bx[q]);
+        bx[q] = fma(-hi.y, pj.y, bx[q]);
+        by[q] = fma(hi.x, pj.y, by[q]);
+        by[q] = fma(hi.y, pj.x, by[q]);
+      }
+      v = cmi(cmk((ax[0] + ax[1]) - (bx[0] + bx[1]), (ay[0] + ay[1]) + (by[0] + by[1])));
+      if (i < nch && j >= nch) v = cadd(v, cmi(cscale(Pe, -a.wx2)));
+    } else if (i == j) {
       double2 beta = cz();
 #pragma unroll
       for (int l = 0; l < N; l++) beta = cadd(beta, cmul(HF(i, l), Pf(i, l)));
@@ -319,7 +370,7 @@ static cudaError_t launch_ep(const DevTables& tb, const DevConsts* cst, const St
     // rows of the k grid one block of KT consecutive k points can touch
     const int rows = (tb.n2 + KT - 2) / tb.n2 + 1;
     const size_t bytes = sizeof(double2) * ((size_t)rows * 2 * tb.ncut * NT + tb.ncut * KT);
-    const size_t static_bytes = sizeof(double2) * 3 * NT * KT;
+    const size_t static_bytes = RowsEP<N, KT>::FULL ? sizeof(double2) * 2 * RowsEP<N, KT>::SIZE + 1024 : sizeof(double2) * 3 * NT * KT;
     if (bytes + static_bytes <= 48 * 1024) {
       b.stage_rows = rows;
       dyn = bytes;
@@ -336,7 +387,7 @@ cudaError_t launch_rhs(const DevTables& tb, const DevConsts* cst, const StageArg
     case 3: return launch_ep<3, 32>(tb, cst, a, s);
     case 4: return launch_ep<4, 32>(tb, cst, a, s);
     case 5: return launch_ep<5, 32>(tb, cst, a, s);
-    case 8: return launch_ep<8, 16>(tb, cst, a, s);
+    case 8: return launch_ep<8, 8>(tb, cst, a, s);
     case 16: return launch_ep<16, 4>(tb, cst, a, s);
     default: return cudaErrorInvalidValue;
   }
