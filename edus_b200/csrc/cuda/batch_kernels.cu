@@ -112,9 +112,15 @@ __device__ __forceinline__ bool field_on(const double* E) {
 //   s=3: P0 = P1 + dt/6 k4                        (field at t + dt)
 // Resident blocks per SM the register budget is sized for: register profile 0
 // aims at about 36 warps per SM (56 registers), profile 1 at 24 warps (up to
-// 80-96 registers, fewer spills). The autotuner picks one per class.
+// 80-96 registers, fewer spills). The autotuner picks one per class. Blocks of
+// 288 threads (8 bands with 8 k points per tile, 16 bands with 2) are three per SM
+// in profile 1: 72 registers hold the row products that spill at profile 0's 56,
+// and a third block covers the barriers of the other two, which two blocks at 96
+// registers do not. FP64, 96 x 96 k points, million k-point steps/s: 8 bands 163
+// against 151 for profile 0 (two blocks: slower than profile 0), 16 bands 27.1
+// against 24.1 with two blocks.
 constexpr int min_blocks(int nthr, int occ) {
-  const int target = occ == 0 ? 1152 : 768;
+  const int target = occ == 0 ? 1152 : (nthr == 288 ? 864 : 768);
   return target / nthr > 0 ? target / nthr : 1;
 }
 
