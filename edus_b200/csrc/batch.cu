@@ -377,7 +377,9 @@ int build_model_tc(edus_batch* b, const Problem& P, const Inst& I) {
   // H and D on the tensor cores; dH/dk, an observable-only table whose k sums
   // cancel strongly, is the reference's stencil over an FP64 H(k) (CUDA cores)
   const int ncomp = 4;
-  const int kp = tc_pad_k(nr), ncols = 2 * ncomp * nt;
+  const TcForm form = tc_gemm_form();
+  const int kp = tc_depth(nr, form), ncols = 2 * ncomp * nt;
+  const size_t csize = tc_c_size(nk, nt, form);
   // upper coefficients of H(R) and the symmetrised dipoles; the scale of a GEMM
   // column is the power of two that brings every value into [-1/2, 1/2)
   std::vector<double2> coef((size_t)ncomp * nt * nr);
@@ -407,7 +409,7 @@ int build_model_tc(edus_batch* b, const Problem& P, const Inst& I) {
   const size_t plane = (size_t)nt * nk;
   const size_t bytes = align256(sizeof(double) * 3 * nk) + align256(sizeof(double) * 3 * nr) + align256(sizeof(double2) * coef.size()) +
                        align256(sizeof(double) * ncols) + align256(sizeof(uint16_t) * (size_t)ncols * kp) + align256(sizeof(double2) * hdr.size()) + align256(sizeof(double) * gb.size()) +
-                       align256(sizeof(uint16_t) * (size_t)nk * kp) + align256(sizeof(double) * (size_t)nk * ncols) +
+                       align256(sizeof(uint16_t) * (size_t)nk * kp) + align256(sizeof(double) * csize) +
                        align256(sizeof(double2) * plane) + align256(sizeof(double2) * n * n * nk) +
                        (I.GE ? align256(sizeof(double2) * plane) + align256(sizeof(double2) * 3 * plane) : 0);
   char* base = nullptr;
@@ -441,10 +443,11 @@ int build_model_tc(edus_batch* b, const Problem& P, const Inst& I) {
   t.Rvec = dR;
   t.coef = dcoef;
   t.colscale = dscale;
-  t.Bw = (uint16_t*)carve(sizeof(uint16_t) * (size_t)ncols * kp);
+  t.op.form = form;
+  t.op.B = (uint16_t*)carve(sizeof(uint16_t) * (size_t)ncols * kp);
   t.hdiagR = dh;
-  t.Aw = (uint16_t*)carve(sizeof(uint16_t) * (size_t)nk * kp);
-  t.Cw = (double*)carve(sizeof(double) * (size_t)nk * ncols);
+  t.op.A = (uint16_t*)carve(sizeof(uint16_t) * (size_t)nk * kp);
+  t.op.C = (double*)carve(sizeof(double) * csize);
   t.H32 = (float2*)I.H;
   t.D32 = (float2*)I.D;
   t.Hdiag = (double*)I.Hdiag;

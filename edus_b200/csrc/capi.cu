@@ -414,7 +414,7 @@ int vg_tables(edus_ctx* c, double t) {
   if (c->vg_tc) {
     for (int i = 0; i < 3; i++) c->vgt.A[i] = c->vga.A[i];
     CK(batch::tc_vg_stage(c->vgt, c->stream));
-    c->launches += 3;
+    c->launches += c->vgt.op.form == batch::TcForm::planes ? 2 : 3;
   } else {
     CK(launch_vg_tables(c->vga, c->stream));
     c->launches++;
@@ -1926,7 +1926,9 @@ int edus_create(const edus_problem* pb, const edus_options* opt, edus_ctx** out)
     if (c->vg_tc) {
       // power-of-two scale of each GEMM column from max_R |c(R)| (bounds |Re|, |Im| of
       // e^{2 pi i A.R} c(R) for every A): every sliced value lies in [-1/2, 1/2]
-      const int ncols = 8 * nt, kpad = batch::tc_pad_k(nr);
+      const batch::TcForm form = batch::tc_gemm_form();
+      const int ncols = 8 * nt, kpad = batch::tc_depth(nr, form);
+      const size_t csize = batch::tc_c_size(nk, nt, form);
       std::vector<double> cs(ncols);
       for (int ce = 0; ce < 4 * nt; ce++) {
         double amax = 0.;
@@ -1937,7 +1939,7 @@ int edus_create(const edus_problem* pb, const edus_options* opt, edus_ctx** out)
       uint16_t *dA = nullptr, *dB = nullptr;
       double* dC = nullptr;
       if ((rc = dalloc(c, &dcs, (size_t)ncols)) || (rc = dalloc(c, &dA, (size_t)nk * kpad)) ||
-          (rc = dalloc(c, &dB, (size_t)ncols * kpad)) || (rc = dalloc(c, &dC, (size_t)nk * ncols)))
+          (rc = dalloc(c, &dB, (size_t)ncols * kpad)) || (csize && (rc = dalloc(c, &dC, csize))))
         return bail(rc);
       if (cudaMemcpyAsync(dcs, cs.data(), sizeof(double) * ncols, cudaMemcpyHostToDevice, c->stream) != cudaSuccess)
         return bail(fail(EDUS_ECUDA, "velocity gauge: upload"));
@@ -1950,15 +1952,14 @@ int edus_create(const edus_problem* pb, const edus_options* opt, edus_ctx** out)
       g.Rvec = dR;
       g.coef = dcoef;
       g.colscale = dcs;
-      g.Aw = dA;
-      g.Bw = dB;
-      g.Cw = dC;
+      g.op.form = form;
+      g.op.A = dA;
+      g.op.B = dB;
+      g.op.C = dC;
       g.H = dH;
       g.D = dD;
       g.err = c->d_err;
       if (batch::tc_vg_prepare(g, c->stream) != cudaSuccess) return bail(fail(EDUS_ECUDA, "velocity gauge: phase slices"));
-      // the TMA tensor maps, unless EDUS_TC_GEMM=cpasync selects the cp.async form
-      if (batch::tc_gemm_tma_wanted()) batch::tc_vg_maps(g);
     }
     c->vg_t = P.t_start;
     if ((rc = vg_tables(c, P.t_start))) return bail(rc);

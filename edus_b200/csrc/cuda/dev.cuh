@@ -84,10 +84,10 @@ __device__ __forceinline__ bool mbar_wait(unsigned long long* bar, uint32_t phas
 // stream retires. pdl_wait() returns once that kernel has completed and its
 // writes are visible; kernels do independent set-up (trig tables into shared
 // memory) before it and touch nothing the previous kernel writes until after
-// it. No kernel triggers its dependents early: measured on the 120 x 120
-// Coulomb step, an early trigger let waiting blocks of the next kernel occupy
-// SM slots and cost 16 %, the implicit trigger at retirement gains 4 %. Both
-// calls are no-ops for a normal launch.
+// it. Only k_bslices, whose grid is resident at once, triggers its dependent
+// early: measured on the 120 x 120 Coulomb step, an early trigger let waiting
+// blocks of the next kernel occupy SM slots and cost 16 %, the implicit trigger
+// at retirement gains 4 %. Both calls are no-ops for a normal launch.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 

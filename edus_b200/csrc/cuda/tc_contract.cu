@@ -14,11 +14,11 @@
 // result is the FP64 sum to about 2^-32 of the terms, so the FP32 tables stored
 // from it equal those of the FP64 CUDA-core build up to the last rounding.
 //
-// Three forms of the GEMM give the same sums bit for bit. k_tc_gemm_ws (the
-// default) and k_tc_gemm_tma (EDUS_TC_GEMM=tma) move 128 x 64 and 64 x 64
-// operand tiles by TMA into 128-byte swizzled stages, four deep, with the
-// loads, MMAs and read-back on separate warps or all issued by thread 0
-// (below). k_tc_gemm (EDUS_TC_GEMM=cpasync): one
+// Three forms of the GEMM give the same planes bit for bit. k_tc_planes (the
+// default) keeps the four slices of each operand once and forms the pair
+// products itself (below). k_tc_gemm_tma (EDUS_TC_GEMM=tma) moves 128 x 64 and
+// 64 x 64 operand tiles by TMA into 128-byte swizzled stages, four deep, all
+// issued by thread 0. k_tc_gemm (EDUS_TC_GEMM=cpasync): one
 // CTA (4 warps) per 128 x 32 tile of C. The 64-deep K slices
 // (128-byte rows of BF16) are staged with cp.async into two shared-memory
 // stages in the K-major canonical layout without swizzle (16-byte chunks of 8
@@ -47,9 +47,10 @@ constexpr int TM = 128, TN = 32, TK = 64;  // CTA tile and K slice (BF16 element
 constexpr int kThreads = 128;
 constexpr uint32_t kTmemCols = 32;
 
-// A' rows: phases of k point m over the R vectors; segment p holds slice
-// tc_pair_a(p) of [cos | sin], zero padded to the segment length. One phase
-// is evaluated once and written to every segment.
+// A' rows: phases of k point m over the R vectors, [cos | sin] zero padded to
+// the segment length. Four segments (kpad = 4 kseg): segment t holds slice t
+// (k_tc_planes forms the pairs itself); ten: segment p holds slice tc_pair_a(p).
+// One phase is evaluated once and written to every segment.
 __global__ void k_phase_split(const double* __restrict__ kpt, const double* __restrict__ Rvec, int nk, int nr, int kseg,
                               int kpad, uint16_t* __restrict__ A) {
   const int m = blockIdx.x;
@@ -66,8 +67,13 @@ __global__ void k_phase_split(const double* __restrict__ kpt, const double* __re
 #pragma unroll
       for (int t = 0; t < kTcSlices; t++) sl[t] = tc_bf16(tc_slice(y, t));  // at most 8 significant bits: exact in BF16
     }
+    if (kpad == kTcSlices * kseg) {
 #pragma unroll
-    for (int p = 0; p < kTcPairs; p++) row[(size_t)p * kseg + q] = sl[tc_pair_a(p)];
+      for (int t = 0; t < kTcSlices; t++) row[(size_t)t * kseg + q] = sl[t];
+    } else {
+#pragma unroll
+      for (int p = 0; p < kTcPairs; p++) row[(size_t)p * kseg + q] = sl[tc_pair_a(p)];
+    }
   }
 }
 
@@ -433,175 +439,255 @@ __global__ void __launch_bounds__(kThreads, 1) k_tc_gemm_tma(const __grid_consta
 }
 
 // ------------------------------------------------------- warp-specialised form
-// The TMA-staged GEMM with its roles on separate warps, so that loads, MMAs and
-// the FP64 read-back of finished segments overlap instead of taking turns on
-// thread 0 between block barriers: warp 4 (one lane) issues the TMA loads of
-// slice s into stage s % 4 once the MMAs of slice s - 4 have released it;
-// warp 5 (one lane) issues the MMAs of slice s once its stage is full, into
-// the TMEM accumulator of its segment's parity, after the read-back of the
-// segment two back has freed that accumulator, and commits them to the
-// stage's "empty" barrier and, at a segment's end, to the accumulator's
-// "full" barrier; warps 0-3 read each finished segment (32 TMEM lanes each)
-// into FP64 registers and arrive on the accumulator's "free" barrier. The
-// sums are those of the other forms, in the same order. Every wait is bounded;
-// a role that times out raises a shared abort flag and stops, the others stop
-// at their next wait, and before TMEM and shared memory are released the
-// producer waits (bounded) for its last loads and the MMA lane for its last
-// commit.
-constexpr int kWsThreads = 192;
+// H and D planes straight from the four slices of each operand. The pair
+// segments of the forms above load every slice up to four times (983 KB per
+// 128 x 64 tile at 121 R vectors), read the accumulator back into FP64
+// registers after every pair, and write C for a second kernel to scatter. Here
+// a 64-deep chunk of all four slices of both operands is loaded once and its
+// ten pair products are formed from shared memory. Pairs of one a + b have the
+// same power of two and share an accumulator: over a group of kGroup3 chunks
+// its sums are at most 4 x 256 = 1024 deep, so they are still exact. The four
+// accumulators are read back once per group (one group up to 128 R vectors) and
+// added in FP64, exact too (25 bits each, 8 bits apart): the results have the
+// bits of the other forms. They go to the planes, lanes along k.
+// Tile 128 x 80: the 288 columns of 8 bands are four tiles, so 64 x 64 k points
+// are 128 CTAs, one wave. A chunk is 104 KB, two of them one CTA's shared
+// memory, whose bandwidth bounds the products: the B slices of a chunk lie one
+// after another, and so do the accumulators, so that slice a of A meets up to
+// three B slices in one MMA (N 160, 160, 240, 160, 80 for a = 0, 0, 1, 2, 3) and
+// is read five times in all instead of ten. Read-back and stores take eight warps
+// and rolled loops: unrolled, their instruction fetches took 40 % of the kernel.
+// 8 bands, 121 R vectors, 64 x 64 k points: 11.1 us (16.4 with one MMA per
+// pair, four read-back warps and unrolled loops); with pair segments and these
+// roles 39.5 us and 6.6 us for the scatter.
+// Roles: warp 8 (one lane) loads a chunk onto two barriers, first what the
+// first MMAs need; warp 9 (one lane) issues the MMAs; warps 0-7 read back 32
+// TMEM lanes and 40 columns each. Every wait is bounded; a role that times out
+// raises a shared abort flag and stops, the others stop at their next wait, and
+// before TMEM and shared memory are released the last loads and the last commit
+// are waited for (bounded).
+constexpr int kWsThreads = 320;
+constexpr int TN3 = 80, kStages3 = 2, kGroup3 = 4, kTmemCols3 = 512;
+constexpr uint32_t kSliceA3 = TM * TK * 2, kSliceB3 = TN3 * TK * 2, kStage3 = kTcSlices * (kSliceA3 + kSliceB3);
+constexpr uint32_t kFirst3 = kSliceA3 + 2 * kSliceB3;  // A slice 0, B slices 0 and 1
+constexpr size_t kPlanesSmem = (size_t)kStages3 * kStage3 + 1024;
+static_assert(kSliceA3 % 1024 == 0 && kSliceB3 % 1024 == 0, "swizzle atoms are 1024 bytes");
+static_assert(kTcSlices * kGroup3 * TK <= 1024, "exact FP32 sums");
+static_assert(kTcSlices == 4 && kTcSlices * TN3 <= kTmemCols3 && 3 * TN3 <= 256 && TN3 % 16 == 0, "MMA shapes");
 
 __device__ __forceinline__ void mbar_arrive(unsigned long long* bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
 
-__global__ void __launch_bounds__(kWsThreads, 2) k_tc_gemm_ws(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB,
-                                                              double* __restrict__ C, int M, int N, int Kp, int kseg, int* err) {
+// T is double2 (velocity gauge) or float2 (batch tables); MULTI: more than one
+// group, whose sums meet in registers
+template <class T, bool MULTI>
+__global__ void __launch_bounds__(kWsThreads, 1) k_tc_planes(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB,
+                                                             T* __restrict__ H, T* __restrict__ D, int nk, int n, int ntri, int kseg,
+                                                             int* err) {
   extern __shared__ __align__(1024) unsigned char smem[];
-  constexpr uint32_t kStageA = TM * TK * 2, kStageB = TN2 * TK * 2, kStage = kStageA + kStageB;
-  __shared__ unsigned long long full[kStages2], empty[kStages2], accf[2], acce[2];
+  __shared__ unsigned long long full[kStages3][2], empty[kStages3], accf, acce;
   __shared__ uint32_t tmem_base;
-  __shared__ int abort_flag, loads_issued, last_commit;
+  __shared__ int abort_flag, loads_issued, commits;
   const int tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
-  const int m0 = blockIdx.x * TM, n0 = blockIdx.y * TN2;
+  const int m0 = blockIdx.x * TM, n0 = blockIdx.y * TN3, N = 8 * ntri;
   if (warp == 0) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base)), "r"(2 * kTmemCols2));
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base)), "r"(kTmemCols3));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
   }
   if (tid == 32) {
-    for (int b = 0; b < kStages2; b++) {
-      mbar_init(&full[b], 1);
+    asm volatile("prefetch.tensormap [%0];" ::"l"(&mapA) : "memory");
+    asm volatile("prefetch.tensormap [%0];" ::"l"(&mapB) : "memory");
+    for (int b = 0; b < kStages3; b++) {
+      mbar_init(&full[b][0], 1);
+      mbar_init(&full[b][1], 1);
       mbar_init(&empty[b], 1);
     }
-    for (int b = 0; b < 2; b++) {
-      mbar_init(&accf[b], 1);
-      mbar_init(&acce[b], 4);  // one arrival per read-back warp
-    }
+    mbar_init(&accf, 1);
+    mbar_init(&acce, 8);  // one arrival per read-back warp
     abort_flag = 0;
     loads_issued = 0;
-    last_commit = -1;
+    commits = 0;
   }
   asm volatile("tcgen05.fence::before_thread_sync;");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;");
   const uint32_t tmem = tmem_base;
   const uint32_t base = (smem_u32(smem) + 1023u) & ~1023u;
-  const int S = Kp / TK, SEG = kseg / TK, P = S / SEG;
+  pdl_wait();  // the coefficient slices; the set-up above overlaps the kernel that cuts them
+  const int chunks = kseg / TK;
   volatile int* abortp = &abort_flag;
-  double acc[TN2];
-#pragma unroll
-  for (int c = 0; c < TN2; c++) acc[c] = 0.;
 
-  if (warp == 4) {
+  if (warp == 8) {
     if (lane == 0) {
-      int s = 0;
-      for (; s < S; s++) {
-        const int st = s % kStages2;
+      int c = 0;
+#pragma unroll 1
+      for (; c < chunks; c++) {
+        const int st = c % kStages3;
         if (*abortp) break;
-        if (s >= kStages2 && !mbar_wait(&empty[st], (uint32_t)(((s / kStages2) - 1) & 1), err)) {
+        if (c >= kStages3 && !mbar_wait(&empty[st], (uint32_t)((c / kStages3 - 1) & 1), err)) {
           *abortp = 1;
           break;
         }
-        const uint32_t sa = base + (uint32_t)st * kStage, sb = sa + kStageA;
-        mbar_expect_tx(&full[st], kStage);
-        tma_load_2d(sa, &mapA, s * TK, m0, smem_u32(&full[st]));
-        tma_load_2d(sb, &mapB, s * TK, n0, smem_u32(&full[st]));
+        const uint32_t sa = base + (uint32_t)st * kStage3, sb = sa + kTcSlices * kSliceA3;
+        mbar_expect_tx(&full[st][0], kFirst3);
+        mbar_expect_tx(&full[st][1], kStage3 - kFirst3);
+#pragma unroll 1
+        for (int q = 0; q < 2 * kTcSlices; q++) {
+          // A0, B0, B1 | B2, B3, A1, A2, A3
+          const bool isA = q == 0 || q > kTcSlices;
+          const int t = isA ? (q == 0 ? 0 : q - kTcSlices) : q - 1;
+          const uint32_t bar = smem_u32(&full[st][q < 3 ? 0 : 1]);
+          if (isA)
+            tma_load_2d(sa + (uint32_t)t * kSliceA3, &mapA, t * kseg + c * TK, m0, bar);
+          else
+            tma_load_2d(sb + (uint32_t)t * kSliceB3, &mapB, t * kseg + c * TK, n0, bar);
+        }
       }
-      loads_issued = s;
+      loads_issued = c;
     }
-  } else if (warp == 5) {
+  } else if (warp == 9) {
     if (lane == 0) {
-      int last = -1;
-      for (int s = 0; s < S; s++) {
-        const int st = s % kStages2, p = s / SEG, buf = p & 1;
+      int c = 0;
+#pragma unroll 1
+      for (; c < chunks; c++) {
+        const int st = c % kStages3;
+        const uint32_t par = (uint32_t)((c / kStages3) & 1);
         if (*abortp) break;
-        if (!mbar_wait(&full[st], (uint32_t)((s / kStages2) & 1), err)) {
-          *abortp = 1;
-          break;
-        }
-        // a segment's first slice reuses the accumulator of the segment two back: wait for its read-back
-        if (s % SEG == 0 && p >= 2 && !mbar_wait(&acce[buf], (uint32_t)(((p / 2) - 1) & 1), err)) {
-          *abortp = 1;
-          break;
-        }
-        asm volatile("tcgen05.fence::after_thread_sync;");
-        const uint32_t sa = base + (uint32_t)st * kStage, sb = sa + kStageA;
-        const uint32_t dtm = tmem + (uint32_t)(buf * kTmemCols2);
+        bool ok = true;
+        // a group reuses the accumulators of the one before: wait for their read-back
+        if (MULTI && c % kGroup3 == 0 && c > 0) ok = mbar_wait(&acce, (uint32_t)((c / kGroup3 - 1) & 1), err);
+        const uint64_t da0 = sw128_desc(base + (uint32_t)st * kStage3);
+        const uint64_t db0 = sw128_desc(base + (uint32_t)st * kStage3 + kTcSlices * kSliceA3);
+#pragma unroll 1
+        for (int p = 0; p <= kTcSlices && ok; p++) {
+          // slice a of A with slices b .. b + nb - 1 of B into accumulators a + b ..
+          const int a = p < 2 ? 0 : p - 1, b = p == 1 ? 2 : 0, nb = p < 2 ? 2 : kTcSlices - a;
+          if (p < 2) ok = mbar_wait(&full[st][p], par, err);
+          if (!ok) break;
+          asm volatile("tcgen05.fence::after_thread_sync;");
+          const uint32_t idesc =
+              (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(nb * (TN3 >> 3)) << 17) | ((uint32_t)(TM >> 4) << 24);
+          const uint32_t dtm = tmem + (uint32_t)((a + b) * TN3);
+          const uint64_t da = da0 + (uint64_t)(a * (kSliceA3 >> 4)), db = db0 + (uint64_t)(b * (kSliceB3 >> 4));
+          const uint32_t first = c % kGroup3 == 0 && p < 2 ? 0u : 1u;  // starts two accumulators
 #pragma unroll
-        for (int j = 0; j < TK / 16; j++) {
-          const uint64_t da = sw128_desc(sa + (uint32_t)(32 * j));
-          const uint64_t db = sw128_desc(sb + (uint32_t)(32 * j));
-          const uint32_t accum = (j > 0 || s % SEG != 0) ? 1u : 0u;
-          asm volatile(
-              "{\n\t.reg .pred p;\n\t"
-              "setp.ne.b32 p, %4, 0;\n\t"
-              "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %6, %7, %8}, p;\n\t}\n" ::"r"(dtm),
-              "l"(da), "l"(db), "r"(kIdesc2), "r"(accum), "r"(0u), "r"(0u), "r"(0u), "r"(0u));
+          for (int j = 0; j < TK / 16; j++) {
+            // K step j: 32 bytes into every 128-byte swizzled row
+            const uint32_t accum = j > 0 ? 1u : first;
+            asm volatile(
+                "{\n\t.reg .pred p;\n\t"
+                "setp.ne.b32 p, %4, 0;\n\t"
+                "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %6, %7, %8}, p;\n\t}\n" ::"r"(dtm),
+                "l"(da + (uint64_t)(2 * j)), "l"(db + (uint64_t)(2 * j)), "r"(idesc), "r"(accum), "r"(0u), "r"(0u), "r"(0u), "r"(0u));
+          }
         }
+        // (also on the way out: what was issued ends before its stage and TMEM are released)
         asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(&empty[st]))
                      : "memory");
-        if (s % SEG == SEG - 1)
-          asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(&accf[buf]))
-                       : "memory");
-        last = s;
+        commits = c + 1;
+        if (!ok) {
+          *abortp = 1;
+          break;
+        }
+        if (c % kGroup3 == kGroup3 - 1 || c == chunks - 1)
+          asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(&accf)) : "memory");
       }
-      last_commit = last;
     }
   } else {
-    // read-back warps: TMEM lanes 32 warp .. 32 warp + 31 are rows m0 + 32 warp + lane
-    for (int p = 0; p < P; p++) {
-      const int buf = p & 1;
-      const bool ok = !*abortp && mbar_wait(&accf[buf], (uint32_t)((p / 2) & 1), err);
+    // warp w: TMEM lanes 32 (w % 4) .. + 31, k points m0 + 32 (w % 4) + lane; columns 40 (w / 4) .. + 39
+    constexpr int kCols = TN3 / 2;
+    const int k = m0 + (warp % 4) * 32 + lane, col0 = (warp / 4) * kCols;
+    const uint32_t trow = tmem + ((uint32_t)((warp % 4) * 32) << 16) + (uint32_t)col0;
+    // column pair 2 ce, 2 ce + 1 = Re, Im of component and element ce = comp * ntri + e: planes
+    // 0 .. ntri - 1 are H, the following D; e's row i of the upper triangle begins at its diagonal
+    // element ed, whose imaginary part is zero (Wannier.h:489-492)
+    int ce = (n0 + col0) / 2, e = ce % ntri, i = 0, ed = 0;
+    while (e >= ed + n - i) ed += n - i++;
+    auto store8 = [&](const double* z) {
+#pragma unroll
+      for (int u = 0; u < 8; u += 2, ce++) {
+        T o;
+        o.x = z[u];
+        o.y = e == ed ? 0. : z[u + 1];
+        if (k < nk && 2 * ce < N) (ce < ntri ? H + (size_t)ce * nk : D + (size_t)(ce - ntri) * nk)[k] = o;
+        if (++e == ed + n - i) ed += n - i++;
+        if (e == ntri) e = i = ed = 0;
+      }
+    };
+    // the four accumulators of columns c0 .. c0 + 7, added to z
+    auto read8 = [&](int c0, double* z) {
+      uint32_t v[kTcSlices][8];
+#pragma unroll
+      for (int t = 0; t < kTcSlices; t++)
+        asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                     : "=r"(v[t][0]), "=r"(v[t][1]), "=r"(v[t][2]), "=r"(v[t][3]), "=r"(v[t][4]), "=r"(v[t][5]), "=r"(v[t][6]),
+                       "=r"(v[t][7])
+                     : "r"(trow + (uint32_t)(t * TN3 + c0)));
+      asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+      for (int t = 0; t < kTcSlices; t++)
+#pragma unroll
+        for (int u = 0; u < 8; u++) z[u] += (double)__uint_as_float(v[t][u]);
+    };
+    auto finished = [&](int g) {
+      const bool ok = !*abortp && mbar_wait(&accf, (uint32_t)(g & 1), err);
       if (__any_sync(0xffffffffu, !ok)) {
         if (lane == 0) *abortp = 1;
-        break;
+        return false;
       }
       asm volatile("tcgen05.fence::after_thread_sync;");
+      return true;
+    };
+    if (!MULTI) {
+      if (finished(0))
+#pragma unroll 1
+        for (int c0 = 0; c0 < kCols; c0 += 8) {
+          double z[8] = {0., 0., 0., 0., 0., 0., 0., 0.};
+          read8(c0, z);
+          store8(z);
+        }
+    } else {
+      const int groups = (chunks + kGroup3 - 1) / kGroup3;
+      double acc[kCols];
 #pragma unroll
-      for (int c0 = 0; c0 < TN2; c0 += 8) {
-        uint32_t v[8];
-        const uint32_t taddr = tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(buf * kTmemCols2 + c0);
-        asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-                     : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
-                     : "r"(taddr));
-        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+      for (int c = 0; c < kCols; c++) acc[c] = 0.;
+      int g = 0;
+      for (; g < groups && finished(g); g++) {
 #pragma unroll
-        for (int u = 0; u < 8; u++) acc[c0 + u] += (double)__uint_as_float(v[u]);
+        for (int c0 = 0; c0 < kCols; c0 += 8) read8(c0, acc + c0);
+        asm volatile("tcgen05.fence::before_thread_sync;");
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&acce);
       }
-      asm volatile("tcgen05.fence::before_thread_sync;");
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&acce[buf]);
+      if (g == groups)
+#pragma unroll
+        for (int c0 = 0; c0 < kCols; c0 += 8) store8(acc + c0);
     }
   }
   __syncthreads();
-  if (!*abortp) {
-    if (warp < 4) {
-      const int row = m0 + warp * 32 + lane;
-      if (row < M)
-#pragma unroll
-        for (int c = 0; c < TN2; c++)
-          if (n0 + c < N) C[(size_t)row * N + n0 + c] = acc[c];
-    }
-  } else if (tid == 128) {
-    // the last loads issued (one per stage at most is outstanding) land before the stages go away
-    for (int s = loads_issued - kStages2 < 0 ? 0 : loads_issued - kStages2; s < loads_issued; s++)
-      mbar_wait(&full[s % kStages2], (uint32_t)((s / kStages2) & 1), err);
-  } else if (tid == 160 && last_commit >= 0) {
-    // the last committed MMAs finish before their TMEM is released
-    mbar_wait(&empty[last_commit % kStages2], (uint32_t)((last_commit / kStages2) & 1), err);
+  if (*abortp) {
+    // the last loads issued (one chunk per stage at most is outstanding) land before the stages go away
+    if (tid == 256)
+      for (int c = loads_issued - kStages3 < 0 ? 0 : loads_issued - kStages3; c < loads_issued; c++)
+        for (int t = 0; t < 2; t++) mbar_wait(&full[c % kStages3][t], (uint32_t)((c / kStages3) & 1), err);
+    // and the last committed MMAs finish before their TMEM is released
+    if (tid == 288 && commits > 0) mbar_wait(&empty[(commits - 1) % kStages3], (uint32_t)(((commits - 1) / kStages3) & 1), err);
   }
   asm volatile("tcgen05.fence::before_thread_sync;");
   __syncthreads();
-  if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(2 * kTmemCols2));
+  if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols3));
 }
 
 // Coefficient slices of c_A(R) = e^{2 pi i A.R} c(R) (velocity gauge; the model
 // build of a batch instance has A = 0, where c_A = c exactly), one thread per
 // (column, K entry); column 2 ce + part holds [Re c_A ; -Im c_A] (part 0) or
 // [Im c_A ; Re c_A] (part 1), divided by the column's scale, cut and pre-multiplied
-// by 2 scale (the phases enter halved). 2.1 us for 8 bands and 121 R vectors; cut
+// by 2 scale (the phases enter halved); segments as in k_phase_split. 2.1 us for 8 bands and 121 R vectors; cut
 // on the host for every admitted instance it was 3 ms of one core.
 __global__ void k_bslices(const double2* __restrict__ coef, const double* __restrict__ Rvec, const double* __restrict__ colscale,
                              double A0, double A1, double A2, int ntri, int nr, int kseg, int kpad, uint16_t* __restrict__ B) {
+  pdl_trigger();
   const int q = blockIdx.x * blockDim.x + threadIdx.x;  // K entry
   const int col = blockIdx.y;                          // 2 (comp * ntri + e) + part
   const int K = 2 * nr;
@@ -616,8 +702,16 @@ __global__ void k_bslices(const double2* __restrict__ coef, const double* __rest
   const double v = part == 0 ? (q < nr ? re : -im) : (q < nr ? im : re);
   const double scale = colscale[col];
   uint16_t* row = B + (size_t)col * kpad;
+  uint16_t sl[kTcSlices];
 #pragma unroll
-  for (int p = 0; p < kTcPairs; p++) row[(size_t)p * kseg + q] = tc_bf16(2.0 * scale * tc_slice(v / scale, tc_pair_b(p)));
+  for (int t = 0; t < kTcSlices; t++) sl[t] = tc_bf16(2.0 * scale * tc_slice(v / scale, t));
+  if (kpad == kTcSlices * kseg) {
+#pragma unroll
+    for (int t = 0; t < kTcSlices; t++) row[(size_t)t * kseg + q] = sl[t];
+  } else {
+#pragma unroll
+    for (int p = 0; p < kTcPairs; p++) row[(size_t)p * kseg + q] = sl[tc_pair_b(p)];
+  }
 }
 
 // C[k][col] -> FP64 planes H [ntri][nk], D [3][ntri][nk]; diagonal imaginary parts zero
@@ -642,33 +736,8 @@ __global__ void k_scatter64(const double* __restrict__ C, int nk, int n, int ntr
 size_t tc_gemm_smem() { return 2 * sizeof(uint16_t) * (TM + TN) * TK + 1024; }
 
 int tc_seg_k(int nr) { return ((2 * nr + TK - 1) / TK) * TK; }
-int tc_pad_k(int nr) { return kTcPairs * tc_seg_k(nr); }
-
-cudaError_t tc_gemm_run(const uint16_t* Aw, const uint16_t* Bw, double* Cw, int M, int ncols, int kpad, int kseg, int* err,
-                        const CUtensorMap* mapA, const CUtensorMap* mapB, cudaStream_t s);
-bool tc_gemm_tma_wanted();
-cudaError_t tc_gemm_maps(const uint16_t* Aw, const uint16_t* Bw, int M, int ncols, int kpad, CUtensorMap* mapA, CUtensorMap* mapB);
-
-cudaError_t tc_contract(const TcArgs& a, cudaStream_t s) {
-  const int kpad = tc_pad_k(a.nr);
-  const int ncols = 8 * a.ntri;
-  k_phase_split<<<a.nk, 256, 0, s>>>(a.kpt, a.Rvec, a.nk, a.nr, tc_seg_k(a.nr), kpad, a.Aw);
-  cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) return e;
-  if ((e = cudaMemsetAsync(a.Bw, 0, sizeof(uint16_t) * (size_t)ncols * kpad, s)) != cudaSuccess) return e;  // segment padding
-  k_bslices<<<dim3((2 * a.nr + 127) / 128, ncols), 128, 0, s>>>(a.coef, a.Rvec, a.colscale, 0., 0., 0., a.ntri, a.nr, tc_seg_k(a.nr),
-                                                               kpad, a.Bw);
-  if ((e = cudaGetLastError()) != cudaSuccess) return e;
-  CUtensorMap mA, mB;
-  const bool tma = tc_gemm_tma_wanted() && tc_gemm_maps(a.Aw, a.Bw, a.nk, ncols, kpad, &mA, &mB) == cudaSuccess;
-  if ((e = tc_gemm_run(a.Aw, a.Bw, a.Cw, a.nk, ncols, kpad, tc_seg_k(a.nr), a.err, tma ? &mA : nullptr, tma ? &mB : nullptr, s)) !=
-      cudaSuccess)
-    return e;
-  k_scatter<<<dim3((a.nk + 255) / 256, 4 * a.ntri), 256, 0, s>>>(a.Cw, a.nk, a.n, a.ntri, ncols, a.H32, a.D32);
-  if ((e = cudaGetLastError()) != cudaSuccess) return e;
-  k_diag64<<<dim3((a.nk + 127) / 128, a.n), 128, 0, s>>>(a.kpt, a.Rvec, a.hdiagR, a.H32, a.nk, a.n, a.nr, a.Hdiag, a.Hused);
-  return cudaGetLastError();
-}
+int tc_depth(int nr, TcForm form) { return (form == TcForm::planes ? kTcSlices : kTcPairs) * tc_seg_k(nr); }
+size_t tc_c_size(int nk, int ntri, TcForm form) { return form == TcForm::planes ? 0 : (size_t)nk * 8 * ntri; }
 
 namespace {
 
@@ -677,14 +746,15 @@ using EncodeTiledFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t
                                    CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 
 EncodeTiledFn encode_fn() {
-  static EncodeTiledFn fn = nullptr;
-  if (!fn) {
+  static const EncodeTiledFn fn = []() -> EncodeTiledFn {
     void* p = nullptr;
     cudaDriverEntryPointQueryResult q;
     if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess &&
         q == cudaDriverEntryPointSuccess)
-      fn = (EncodeTiledFn)p;
-  }
+      return (EncodeTiledFn)p;
+    cudaGetLastError();
+    return nullptr;
+  }();
   return fn;
 }
 
@@ -704,80 +774,87 @@ cudaError_t encode_operand(CUtensorMap* map, const uint16_t* ptr, int rows, int 
 
 size_t tma_gemm_smem() { return (size_t)kStages2 * (TM + TN2) * TK * 2 + 1024; }
 
-}  // namespace
-
-cudaError_t tc_vg_prepare(const TcVgArgs& a, cudaStream_t s) {
-  const int kpad = tc_pad_k(a.nr);
-  k_phase_split<<<a.nk, 256, 0, s>>>(a.kpt, a.Rvec, a.nk, a.nr, tc_seg_k(a.nr), kpad, a.Aw);
-  cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) return e;
-  if ((e = cudaMemsetAsync(a.Bw, 0, sizeof(uint16_t) * (size_t)8 * a.ntri * kpad, s)) != cudaSuccess) return e;
-  const size_t smem = std::max(tc_gemm_smem(), (size_t)56 * 1024);
-  if ((e = cudaFuncSetAttribute(k_tc_gemm, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) != cudaSuccess) return e;
-  if ((e = cudaFuncSetAttribute(k_tc_gemm_ws, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tma_gemm_smem())) != cudaSuccess) return e;
-  return cudaFuncSetAttribute(k_tc_gemm_tma, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tma_gemm_smem());
+void launch_scatter(const double* C, int nk, int n, int ntri, float2* H, float2* D, cudaStream_t s) {
+  k_scatter<<<dim3((nk + 255) / 256, 4 * ntri), 256, 0, s>>>(C, nk, n, ntri, 8 * ntri, H, D);
+}
+void launch_scatter(const double* C, int nk, int n, int ntri, double2* H, double2* D, cudaStream_t s) {
+  k_scatter64<<<dim3((nk + 255) / 256, 4 * ntri), 256, 0, s>>>(C, nk, n, ntri, 8 * ntri, H, D);
 }
 
-// GEMM form: the warp-specialised TMA form by default (76.8 us against 110 us
-// for the single-issuer TMA form and 229 us for the cp.async form on the 96 x 96
-// 8-band contraction); EDUS_TC_GEMM=tma selects the single-issuer TMA form,
-// EDUS_TC_GEMM=cpasync the cp.async form (all three give bit-identical sums:
-// every segment's FP32 sums are exact).
-int tc_gemm_form() {
-  const char* form = std::getenv("EDUS_TC_GEMM");
-  if (form && std::strcmp(form, "cpasync") == 0) return 0;
-  if (form && std::strcmp(form, "tma") == 0) return 1;
-  return 2;
-}
-bool tc_gemm_tma_wanted() { return tc_gemm_form() != 0; }
-
-cudaError_t tc_gemm_maps(const uint16_t* Aw, const uint16_t* Bw, int M, int ncols, int kpad, CUtensorMap* mapA, CUtensorMap* mapB) {
-  cudaError_t e = encode_operand(mapA, Aw, M, kpad, TM);
-  if (e == cudaSuccess) e = encode_operand(mapB, Bw, ncols, kpad, TN2);
-  return e;
-}
-
-// C = A' B'^T over the slice-pair segments: the TMA form with the given tensor maps, else the cp.async form
-cudaError_t tc_gemm_run(const uint16_t* Aw, const uint16_t* Bw, double* Cw, int M, int ncols, int kpad, int kseg, int* err,
-                        const CUtensorMap* mapA, const CUtensorMap* mapB, cudaStream_t s) {
+// H and D planes from A' and B' in the layout of o.form
+template <class T>
+cudaError_t gemm_planes(const TcOperands& o, T* H, T* D, int nk, int n, int ntri, int nr, int* err, cudaStream_t s) {
+  const int ncols = 8 * ntri, kpad = tc_depth(nr, o.form), kseg = tc_seg_k(nr);
   cudaError_t e;
-  if (mapA && mapB && tc_gemm_form() == 2) {
-    if ((e = cudaFuncSetAttribute(k_tc_gemm_ws, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tma_gemm_smem())) != cudaSuccess)
-      return e;
-    dim3 grid((M + TM - 1) / TM, (ncols + TN2 - 1) / TN2);
-    k_tc_gemm_ws<<<grid, kWsThreads, tma_gemm_smem(), s>>>(*mapA, *mapB, Cw, M, ncols, kpad, kseg, err);
-  } else if (mapA && mapB) {
+  if (o.form == TcForm::planes) {
+    auto kern = kseg > kGroup3 * TK ? k_tc_planes<T, true> : k_tc_planes<T, false>;
+    if ((e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPlanesSmem)) != cudaSuccess) return e;
+    return launch_pdl(kern, dim3((nk + TM - 1) / TM, (ncols + TN3 - 1) / TN3), dim3(kWsThreads), kPlanesSmem, s, o.mapA, o.mapB, H, D, nk, n,
+                      ntri, kseg, err);
+  }
+  if (o.form == TcForm::tma) {
     if ((e = cudaFuncSetAttribute(k_tc_gemm_tma, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tma_gemm_smem())) != cudaSuccess)
       return e;
-    dim3 grid((M + TM - 1) / TM, (ncols + TN2 - 1) / TN2);
-    k_tc_gemm_tma<<<grid, kThreads, tma_gemm_smem(), s>>>(*mapA, *mapB, Cw, M, ncols, kpad, kseg, err);
+    k_tc_gemm_tma<<<dim3((nk + TM - 1) / TM, (ncols + TN2 - 1) / TN2), kThreads, tma_gemm_smem(), s>>>(o.mapA, o.mapB, o.C, nk, ncols, kpad,
+                                                                                                      kseg, err);
   } else {
     // about 55 KB of shared memory per CTA keeps at most four CTAs (256 of the 512 TMEM columns) per SM
     const size_t smem = std::max(tc_gemm_smem(), (size_t)56 * 1024);
     if ((e = cudaFuncSetAttribute(k_tc_gemm, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) != cudaSuccess) return e;
-    dim3 grid((M + TM - 1) / TM, (ncols + TN - 1) / TN);
-    k_tc_gemm<<<grid, kThreads, smem, s>>>(Aw, Bw, Cw, M, ncols, kpad, kseg, err);
+    k_tc_gemm<<<dim3((nk + TM - 1) / TM, (ncols + TN - 1) / TN), kThreads, smem, s>>>(o.A, o.B, o.C, nk, ncols, kpad, kseg, err);
   }
+  if ((e = cudaGetLastError()) != cudaSuccess) return e;
+  launch_scatter(o.C, nk, n, ntri, H, D, s);
   return cudaGetLastError();
 }
 
-cudaError_t tc_vg_maps(TcVgArgs& a) {
-  const cudaError_t e = tc_gemm_maps(a.Aw, a.Bw, a.nk, 8 * a.ntri, tc_pad_k(a.nr), &a.mapA, &a.mapB);
-  a.tma = e == cudaSuccess;
+// phase slices of the grid, zero segment padding of the coefficient slices, tensor maps
+cudaError_t prepare(TcOperands& o, const double* kpt, const double* Rvec, int nk, int ntri, int nr, cudaStream_t s) {
+  const int kpad = tc_depth(nr, o.form), ncols = 8 * ntri;
+  k_phase_split<<<nk, 256, 0, s>>>(kpt, Rvec, nk, nr, tc_seg_k(nr), kpad, o.A);
+  cudaError_t e = cudaGetLastError();
+  if (e == cudaSuccess) e = cudaMemsetAsync(o.B, 0, sizeof(uint16_t) * (size_t)ncols * kpad, s);
+  if (e == cudaSuccess && o.form != TcForm::cpasync) e = encode_operand(&o.mapA, o.A, nk, kpad, TM);
+  if (e == cudaSuccess && o.form != TcForm::cpasync) e = encode_operand(&o.mapB, o.B, ncols, kpad, o.form == TcForm::planes ? TN3 : TN2);
   return e;
 }
 
-cudaError_t tc_vg_stage(const TcVgArgs& a, cudaStream_t s) {
-  const int kpad = tc_pad_k(a.nr), kseg = tc_seg_k(a.nr), ncols = 8 * a.ntri;
-  k_bslices<<<dim3((2 * a.nr + 127) / 128, ncols), 128, 0, s>>>(a.coef, a.Rvec, a.colscale, a.A[0], a.A[1], a.A[2], a.ntri,
-                                                                   a.nr, kseg, kpad, a.Bw);
-  cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) return e;
-  if ((e = tc_gemm_run(a.Aw, a.Bw, a.Cw, a.nk, ncols, kpad, kseg, a.err, a.tma ? &a.mapA : nullptr, a.tma ? &a.mapB : nullptr, s)) !=
-      cudaSuccess)
-    return e;
-  k_scatter64<<<dim3((a.nk + 255) / 256, 4 * a.ntri), 256, 0, s>>>(a.Cw, a.nk, a.n, a.ntri, ncols, a.H, a.D);
+cudaError_t cut_coefficients(const TcOperands& o, const double2* coef, const double* Rvec, const double* colscale, const double A[3], int ntri,
+                             int nr, cudaStream_t s) {
+  k_bslices<<<dim3((2 * nr + 127) / 128, 8 * ntri), 128, 0, s>>>(coef, Rvec, colscale, A[0], A[1], A[2], ntri, nr, tc_seg_k(nr),
+                                                                tc_depth(nr, o.form), o.B);
   return cudaGetLastError();
+}
+
+}  // namespace
+
+// The warp-specialised form unless EDUS_TC_GEMM selects another (or the driver
+// has no tensor maps: cp.async). 64 x 64 k points, 8 bands: 11.1 us against
+// 61.9 us for the single-issuer TMA form and 93 us for the cp.async form,
+// scatter included; all three give bit-identical planes (every FP32 sum is exact).
+TcForm tc_gemm_form() {
+  const char* form = std::getenv("EDUS_TC_GEMM");
+  if ((form && std::strcmp(form, "cpasync") == 0) || !encode_fn()) return TcForm::cpasync;
+  if (form && std::strcmp(form, "tma") == 0) return TcForm::tma;
+  return TcForm::planes;
+}
+
+cudaError_t tc_contract(TcArgs& a, cudaStream_t s) {
+  const double zero[3] = {0., 0., 0.};
+  cudaError_t e = prepare(a.op, a.kpt, a.Rvec, a.nk, a.ntri, a.nr, s);
+  if (e == cudaSuccess) e = cut_coefficients(a.op, a.coef, a.Rvec, a.colscale, zero, a.ntri, a.nr, s);
+  if (e == cudaSuccess) e = gemm_planes(a.op, a.H32, a.D32, a.nk, a.n, a.ntri, a.nr, a.err, s);
+  if (e != cudaSuccess) return e;
+  k_diag64<<<dim3((a.nk + 127) / 128, a.n), 128, 0, s>>>(a.kpt, a.Rvec, a.hdiagR, a.H32, a.nk, a.n, a.nr, a.Hdiag, a.Hused);
+  return cudaGetLastError();
+}
+
+cudaError_t tc_vg_prepare(TcVgArgs& a, cudaStream_t s) { return prepare(a.op, a.kpt, a.Rvec, a.nk, a.ntri, a.nr, s); }
+
+cudaError_t tc_vg_stage(const TcVgArgs& a, cudaStream_t s) {
+  cudaError_t e = cut_coefficients(a.op, a.coef, a.Rvec, a.colscale, a.A, a.ntri, a.nr, s);
+  if (e == cudaSuccess) e = gemm_planes(a.op, a.H, a.D, a.nk, a.n, a.ntri, a.nr, a.err, s);
+  return e;
 }
 
 }  // namespace batch

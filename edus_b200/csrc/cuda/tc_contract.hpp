@@ -10,16 +10,31 @@
 namespace edus {
 namespace batch {
 
+// GEMM forms (tc_contract.cu): `planes` has one K segment per slice in A and B and
+// writes the planes itself, the others one per slice pair and a result C.
+enum class TcForm { planes, tma, cpasync };
+TcForm tc_gemm_form();
+int tc_seg_k(int nr);                                   // K segment length: 2 nr padded to the 64-deep K slice
+int tc_depth(int nr, TcForm form);                      // row length of A and B
+size_t tc_c_size(int nk, int ntri, TcForm form);        // doubles in C
+
+// Operands and scratch of a contraction, laid out for `form`
+struct TcOperands {
+  TcForm form = TcForm::cpasync;
+  uint16_t* A = nullptr;  // [nk][tc_depth] phase slices (BF16)
+  uint16_t* B = nullptr;  // [8 ntri][tc_depth] coefficient slices (BF16)
+  double* C = nullptr;    // [nk][8 ntri], none for `planes`
+  CUtensorMap mapA{}, mapB{};
+};
+
 struct TcArgs {
   int n, ntri, nk, nr;
   const double* kpt;     // [nk][3]
   const double* Rvec;    // [nr][3]
   const double2* coef;   // [4][ntri][nr]: H(R), (r_x(R) + r_x(R)^T) / 2 upper entries
   const double* colscale;  // [8 ntri] power-of-two scale of each GEMM column
-  uint16_t* Bw;          // scratch [8 ntri][Kp] coefficient slices (BF16), one K segment per slice pair
   const double2* hdiagR; // [n][nr] H_ii(R) for the FP64 band energies
-  uint16_t* Aw;          // scratch [nk][Kp] phase slices (BF16), one K segment per slice pair
-  double* Cw;            // scratch [nk][8 ntri] GEMM result (FP64 sum of FP32 slices)
+  TcOperands op;
   float2* H32;           // out [ntri][nk]
   float2* D32;           // out [3][ntri][nk]
   double* Hdiag;         // out [n][nk] FP64 band energies
@@ -32,7 +47,7 @@ struct TcArgs {
 // [-1/2, 1/2] and is cut into kTcSlices slices of at most 8 significant bits,
 // slice s a multiple of 2^-(8 s + 8) and at most 128 in magnitude:
 // y = sum_s slice_s(y) + O(2^-33); every slice is exact in BF16. The GEMM runs
-// one K segment per slice pair
+// one K segment per slice pair (or per value of a + b)
 // (a, b) with a + b < kTcSlices; inside a segment every product is an integer
 // times one power of two, at most 2^14 in magnitude, so the tensor core's FP32
 // sums over a segment of up to 1024 are exact and the FP64 sum of the segments
@@ -64,17 +79,14 @@ __host__ __device__ inline uint16_t tc_bf16(double v) {
   memcpy(&u, &f, 4);
   return (uint16_t)(u >> 16);
 }
-// K segment length (2 nr padded to the 64-deep K slice) and the GEMM depth
-int tc_seg_k(int nr);
-int tc_pad_k(int nr);
-cudaError_t tc_contract(const TcArgs& a, cudaStream_t s);
+cudaError_t tc_contract(TcArgs& a, cudaStream_t s);
 
 // Velocity gauge on the tensor cores: H(k + A), D(k + A) of every k point for
 // every RK4 stage as the exact-slice GEMM above. The phase slices of the grid
 // (A' = [cos | sin](2 pi k.R) / 2) are cut once; each stage cuts the
 // coefficient slices of c_A(R) = e^{2 pi i A.R} c(R) on the device (column
 // scales fixed from |c(R)|, which bounds |Re c_A| and |Im c_A| for every A),
-// runs the GEMM and scatters FP64 planes (diagonal imaginary parts zero).
+// runs the GEMM into FP64 planes (diagonal imaginary parts zero).
 struct TcVgArgs {
   int n = 0, ntri = 0, nk = 0, nr = 0;
   const double* kpt = nullptr;       // [nk][3]
@@ -82,22 +94,12 @@ struct TcVgArgs {
   const double2* coef = nullptr;     // [4][ntri][nr]: H(R), (r_x(R) + r_x(R)^T) / 2 upper entries
   const double* colscale = nullptr;  // [8 ntri] power-of-two scale of each GEMM column
   double A[3] = {0, 0, 0};           // crystal coordinates
-  uint16_t* Aw = nullptr;            // [nk][Kp] phase slices (tc_vg_prepare)
-  uint16_t* Bw = nullptr;            // [8 ntri][Kp] coefficient slices (zero padded once)
-  double* Cw = nullptr;              // [nk][8 ntri]
+  TcOperands op;                     // phase slices and segment padding set by tc_vg_prepare
   double2* H = nullptr;              // out [ntri][nk]
   double2* D = nullptr;              // out [3][ntri][nk]
   int* err = nullptr;                // device error word (bounded waits)
-  // TMA descriptors of Aw and Bw (tc_vg_maps); without them the cp.async form runs
-  bool tma = false;
-  CUtensorMap mapA{}, mapB{};
 };
-cudaError_t tc_vg_prepare(const TcVgArgs& a, cudaStream_t s);
-// Encode the TMA descriptors of a.Aw, a.Bw (sets a.tma on success).
-cudaError_t tc_vg_maps(TcVgArgs& a);
-// A TMA-staged GEMM form (warp-specialised by default, single-issuer with
-// EDUS_TC_GEMM=tma) is used unless EDUS_TC_GEMM=cpasync.
-bool tc_gemm_tma_wanted();
+cudaError_t tc_vg_prepare(TcVgArgs& a, cudaStream_t s);
 cudaError_t tc_vg_stage(const TcVgArgs& a, cudaStream_t s);
 
 }  // namespace batch
