@@ -376,7 +376,7 @@ int observe(edus_ctx* c) {
   // velocity gauge: the populations in the eigenbasis of H(k + A) and J1 from
   // the stencil gradient of H(k + A), as with a renormalised H
   const double2* hr = c->vg ? c->vga.H : (c->coul ? c->d_hr : nullptr);
-  CK(launch_observables(c->tb, c->d_cst, c->d_P0, hr, c->d_uev, c->P.p.current, c->P.p.tabs, c->d_part, c->d_done, scaleJ, scaleTA,
+  CK(launch_observables(c->tb, c->d_cst, c->d_P0, hr, c->coul, c->d_uev, c->P.p.current, c->P.p.tabs, c->d_part, c->d_done, scaleJ, scaleTA,
                         rec, slot, c->d_ncond, c->d_pcmax, c->stream));
   c->launches += hr && c->d_uev ? 2 : 1;
   c->nlog++;
@@ -705,7 +705,7 @@ int dyn_enqueue_chunk(edus_ctx* c, int K, bool every) {
       const double scaleTA = std::fabs(c->P.jac) * c->P.dk[0] * c->P.dk[1] * c->P.dk[2];
       edus_obs rec;
       memset(&rec, 0, sizeof(rec));
-      CK(launch_observables(c->tb, c->d_cst, c->d_P0, c->coul ? c->d_hr : nullptr, c->d_uev, c->P.p.current, c->P.p.tabs, c->d_part,
+      CK(launch_observables(c->tb, c->d_cst, c->d_P0, c->coul ? c->d_hr : nullptr, c->coul, c->d_uev, c->P.p.current, c->P.p.tabs, c->d_part,
                             c->d_done, scaleJ, scaleTA, rec, c->d_log, c->d_ncond, c->d_pcmax, c->stream, d));
       c->launches++;
       if (c->snap_on && c->d_snap) {
@@ -2275,7 +2275,7 @@ int edus_observables(edus_ctx* c, edus_obs* out) {
   edus_obs* tmp = c->d_obs_one;
   double scaleJ = c->P.dk[0] * c->P.dk[1] * c->P.dk[2] / c->P.det_a;
   double scaleTA = std::fabs(c->P.jac) * c->P.dk[0] * c->P.dk[1] * c->P.dk[2];
-  CK(launch_observables(c->tb, c->d_cst, c->d_P0, c->vg ? c->vga.H : (c->coul ? c->d_hr : nullptr), c->d_uev, c->P.p.current, c->P.p.tabs, c->d_part,
+  CK(launch_observables(c->tb, c->d_cst, c->d_P0, c->vg ? c->vga.H : (c->coul ? c->d_hr : nullptr), c->coul, c->d_uev, c->P.p.current, c->P.p.tabs, c->d_part,
                         c->d_done, scaleJ, scaleTA, rec, tmp, nullptr, nullptr, c->stream));
   CK(cudaMemcpyAsync(out, tmp, sizeof(edus_obs), cudaMemcpyDeviceToHost, c->stream));
   CK(cudaStreamSynchronize(c->stream));
@@ -2469,7 +2469,7 @@ extern "C" int edus_observables_static(edus_ctx* c, edus_obs* out) {
   rec.dt = c->dt;
   double scaleJ = c->P.dk[0] * c->P.dk[1] * c->P.dk[2] / c->P.det_a;
   double scaleTA = std::fabs(c->P.jac) * c->P.dk[0] * c->P.dk[1] * c->P.dk[2];
-  CK(launch_observables(c->tb, c->d_cst, c->d_P0, c->vg ? c->vga.H : (c->coul ? c->d_hr : nullptr), c->d_uev, c->P.p.current, c->P.p.tabs, base, done,
+  CK(launch_observables(c->tb, c->d_cst, c->d_P0, c->vg ? c->vga.H : (c->coul ? c->d_hr : nullptr), c->coul, c->d_uev, c->P.p.current, c->P.p.tabs, base, done,
                         scaleJ, scaleTA, rec, rec_dev, nullptr, nullptr, c->stream));
   CK(cudaMemcpyAsync(out, rec_dev, sizeof(edus_obs), cudaMemcpyDeviceToHost, c->stream));
   CK(cudaStreamSynchronize(c->stream));

@@ -75,9 +75,10 @@ size_t obs_part_bytes();
 // Complex entries of the eigenvector scratch an instant with a renormalised H
 // needs (0 where the eigenvectors stay in registers).
 size_t obs_eig_count(int n, int nk);
-// hr: renormalised H (null: the model's H, U and dH/dk); uev: its eigenvector
+// hr: renormalised H (null: the model's H, U and dH/dk), by the Coulomb mean
+// field or the velocity gauge; uev: its eigenvector
 // scratch of obs_eig_count entries (null where that is 0 or hr is null).
-cudaError_t launch_observables(const DevTables& tb, const DevConsts* cst, const double2* rho, const double2* hr, double2* uev,
+cudaError_t launch_observables(const DevTables& tb, const DevConsts* cst, const double2* rho, const double2* hr, bool coulomb, double2* uev,
                                int want_current, int want_tabs, void* part, unsigned int* done, double scaleJ,
                                double scaleTA, const ObsRecord& rec, ObsRecord* log, double* ncond_dev,
                                double* pcmax_dev, cudaStream_t s, const DynStep* dyn = nullptr);

@@ -452,7 +452,8 @@ __global__ void __launch_bounds__(ObsEl<N>::THREADS) k_obs_el(DevTables tb, cons
 }
 
 // Rows U[c][i] = conj(Z[i][c]) of the eigenvectors of hr at every k: out[n * n][nk].
-template <int N>
+// WAVE: disjoint rotations together (eig.cuh).
+template <int N, bool WAVE>
 __global__ void __launch_bounds__(128) k_eig_rows(int nk, const double2* __restrict__ hr, double2* __restrict__ out,
                                                   const DynStep* __restrict__ dyn) {
   constexpr int LD = EigGroup<N>::LD, M = 128 / N;
@@ -470,7 +471,10 @@ __global__ void __launch_bounds__(128) k_eig_rows(int nk, const double2* __restr
   }
   __syncthreads();
   double2* A = sm + m * EigGroup<N>::WORDS;
-  eig_herm_group<N>(A, A + N * LD, r);
+  if (WAVE)
+    eig_herm_wave<N>(A, A + N * LD, r);
+  else
+    eig_herm_group<N>(A, A + N * LD, r);
   __syncthreads();
   for (int t = threadIdx.x; t < M * N * N; t += 128) {
     const int mk = t % M, ij = t / M, i = ij / N, j = ij % N;
@@ -484,14 +488,15 @@ cudaError_t launch_obs_n(const DevTables& tb, const DevConsts* cst, const ObsArg
 }
 
 template <int N>
-cudaError_t launch_obs_el(const DevTables& tb, const DevConsts* cst, ObsArgs a, double2* uev, cudaStream_t s) {
+cudaError_t launch_obs_el(const DevTables& tb, const DevConsts* cst, ObsArgs a, double2* uev, bool coulomb, cudaStream_t s) {
   if (a.hr) {
     if (!uev) return cudaErrorInvalidValue;
     constexpr int M = 128 / N;
     constexpr size_t smem = sizeof(double2) * EigGroup<N>::WORDS * M;
     cudaError_t e = cudaSuccess;
-    if (smem > 48 * 1024) e = cudaFuncSetAttribute(k_eig_rows<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e == cudaSuccess) e = launch_pdl(k_eig_rows<N>, dim3((tb.nk + M - 1) / M), dim3(128), smem, s, tb.nk, a.hr, uev, a.dyn);
+    auto eig = coulomb ? k_eig_rows<N, false> : k_eig_rows<N, true>;
+    if (smem > 48 * 1024) e = cudaFuncSetAttribute(eig, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e == cudaSuccess) e = launch_pdl(eig, dim3((tb.nk + M - 1) / M), dim3(128), smem, s, tb.nk, a.hr, uev, a.dyn);
     if (e != cudaSuccess) return e;
     a.uev = uev;
   }
@@ -509,7 +514,7 @@ int obs_parts(int nk) {
 size_t obs_part_bytes() { return sizeof(ObsPart); }
 size_t obs_eig_count(int n, int nk) { return n >= 8 ? (size_t)n * n * nk : 0; }
 
-cudaError_t launch_observables(const DevTables& tb, const DevConsts* cst, const double2* rho, const double2* hr, double2* uev,
+cudaError_t launch_observables(const DevTables& tb, const DevConsts* cst, const double2* rho, const double2* hr, bool coulomb, double2* uev,
                                int want_current, int want_tabs, void* part, unsigned int* done, double scaleJ,
                                double scaleTA, const ObsRecord& rec, ObsRecord* log, double* ncond_dev,
                                double* pcmax_dev, cudaStream_t s, const DynStep* dyn) {
@@ -535,8 +540,8 @@ cudaError_t launch_observables(const DevTables& tb, const DevConsts* cst, const 
     case 3: return launch_obs_n<3>(tb, cst, a, s);
     case 4: return launch_obs_n<4>(tb, cst, a, s);
     case 5: return launch_obs_n<5>(tb, cst, a, s);
-    case 8: return launch_obs_el<8>(tb, cst, a, uev, s);
-    case 16: return launch_obs_el<16>(tb, cst, a, uev, s);
+    case 8: return launch_obs_el<8>(tb, cst, a, uev, coulomb, s);
+    case 16: return launch_obs_el<16>(tb, cst, a, uev, coulomb, s);
     default: return cudaErrorInvalidValue;
   }
 }
