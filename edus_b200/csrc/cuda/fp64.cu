@@ -107,6 +107,23 @@ __global__ void __launch_bounds__(kModeThreads) k_coul_modes(const double2* __re
     mbar_expect_tx(&bar, 2 * col_bytes + trig_bytes);
     bulk_g2s(tc, t1P, trig_bytes, &bar);
   }
+  // so are the coefficients of m = threadIdx.x (5.9 us with their loads behind the
+  // sums below, 5.5 so; 120 x 120 k points, 20 x 20 modes, 3 bands)
+  const bool dg = is_diag[e];
+  double2 c0[4], x0[4];
+  auto coefs = [&](int m) {
+    const size_t mm = (size_t)m * ncut + n, cc = (size_t)ncut * ncut;
+    c0[0] = cA[mm * ntri + e];
+    c0[3] = cD[mm * ntri + e];
+    if (!dg) {
+      c0[1] = cB[mm * ntri + e];
+      c0[2] = cC[mm * ntri + e];
+    }
+    if (X0)
+#pragma unroll
+      for (int q = 0; q < 4; q++) x0[q] = X0[(q * cc + mm) * ntri + e];
+  };
+  if ((int)threadIdx.x < ncut) coefs(threadIdx.x);
   pdl_wait();
   if (threadIdx.x == 0) {
     bulk_g2s(gc, g + ((size_t)n * ntri + e) * n1, col_bytes, &bar);
@@ -135,23 +152,23 @@ __global__ void __launch_bounds__(kModeThreads) k_coul_modes(const double2* __re
     f[o] = cmk((ax + bx) * sc, (ay + by) * sc);
   }
   __syncthreads();
-  const bool dg = is_diag[e];
   for (int m = threadIdx.x; m < ncut; m += kModeThreads) {
     const size_t mm = (size_t)m * ncut + n;
-    const double2 A = cA[mm * ntri + e], D = cD[mm * ntri + e];
+    if (m >= kModeThreads) coefs(m);
+    const double2 A = c0[0], D = c0[3];
     const double2 fcc = f[0 * ncut + m], fcs = f[1 * ncut + m], fsc = f[2 * ncut + m], fss = f[3 * ncut + m];
     double2 xcc = cadd(cmul(A, fcc), cmul(D, fss));
     double2 xcs = csub(cmul(A, fcs), cmul(D, fsc));
     double2 xsc = csub(cmul(A, fsc), cmul(D, fcs));
     double2 xss = cadd(cmul(A, fss), cmul(D, fcc));
     if (X0) {
-      xcc = csub(xcc, X0[(0 * ncut * ncut + mm) * ntri + e]);
-      xcs = csub(xcs, X0[(1 * ncut * ncut + mm) * ntri + e]);
-      xsc = csub(xsc, X0[(2 * ncut * ncut + mm) * ntri + e]);
-      xss = csub(xss, X0[(3 * ncut * ncut + mm) * ntri + e]);
+      xcc = csub(xcc, x0[0]);
+      xcs = csub(xcs, x0[1]);
+      xsc = csub(xsc, x0[2]);
+      xss = csub(xss, x0[3]);
     }
     if (!dg) {
-      const double2 B = cB[mm * ntri + e], C = cC[mm * ntri + e];
+      const double2 B = c0[1], C = c0[2];
       xcc = cadd(xcc, cadd(cmul(B, fcs), cmul(C, fsc)));
       xcs = cadd(xcs, csub(cmul(C, fss), cmul(B, fcc)));
       xsc = cadd(xsc, csub(cmul(B, fss), cmul(C, fcc)));

@@ -54,7 +54,9 @@ struct RowsEP {
   // threads (8 k points; 62.3 us a step on 96 x 96), against 73.8 for two of 576 and
   // 73.5 for four of 288, which spill, and 87.6 for one of 576 as the element-parallel
   // form ran. 16 bands: one block of 544 (51.3 us on 30 x 34; two 53.8, three 68.6).
-  static constexpr int BLOCKS = N == 8 ? 3 : (N == 16 ? 1 : 1);
+  // 3 bands: four blocks of 192 (80 registers, no spills), so that 120 x 120 k points,
+  // 450 blocks, are one wave and not two of 296.
+  static constexpr int BLOCKS = N == 8 ? 3 : (N == 3 ? 4 : 1);
 };
 
 // DYN: the stage scalars come from the adaptive step's device copy (a.dyn);
@@ -69,6 +71,7 @@ __global__ void __launch_bounds__(KT* TriEP<N>::NT, RowsEP<N, KT>::BLOCKS) k_rhs
   __shared__ double2 sHu[FULL ? 1 : NT][KT];  // H~_ij, i <= j
   __shared__ double2 sHl[FULL ? 1 : NT][KT];  // H~_ji, i <= j (D is symmetric, H Hermitian)
   __shared__ double2 fP[Rows::SIZE], fH[Rows::SIZE];  // full matrices
+  __shared__ double sF[kMaxNb][3];  // w_b E_pump,x b_x of the stencil vectors in use
   extern __shared__ double2 dyn[];  // Coulomb row tables: h rows [nrows][2][ncut][NT], trig [2][ncut][KT]
   const int kl = threadIdx.x, e = threadIdx.y;
   const int k0 = blockIdx.x * KT;
@@ -82,22 +85,18 @@ __global__ void __launch_bounds__(KT* TriEP<N>::NT, RowsEP<N, KT>::BLOCKS) k_rhs
   const bool staged = tb.h && a.stage_rows > 0;
   if (staged) {
     // the k2 trig values do not depend on the previous kernel: gathered before
-    // the wait; the inverse-transform rows this block touches (written by the
+    // the wait (an element's threads take the cosines and sines of their own k: no
+    // divisions, which were a quarter of the kernel); the inverse-transform rows this block touches (written by the
     // previous kernel) then arrive by one bulk copy while the threads load
     // their own planes
     const int n2 = tb.n2, nc = tb.ncut;
-    const int tid = threadIdx.y * KT + threadIdx.x, nthr = KT * NT;
     double* ts = reinterpret_cast<double*>(dyn + a.stage_rows * 2 * nc * NT);
-#pragma unroll 4
-    for (int t = tid; t < 2 * nc * KT; t += nthr) {
-      const int q = t % KT, cm = t / KT, cs = cm / nc, m = cm - cs * nc;
-      const int kk = min(k0 + q, nk - 1);
-      const int i2 = kk - (kk / n2) * n2;
-      ts[t] = __ldg((cs == 0 ? tb.t2c : tb.t2s) + m * n2 + i2);
-    }
+    const int i2 = min(k, nk - 1) % n2;
+#pragma unroll 8
+    for (int cm = e; cm < 2 * nc; cm += NT) ts[cm * KT + kl] = __ldg((cm < nc ? tb.t2c + cm * n2 : tb.t2s + (cm - nc) * n2) + i2);
     pdl_wait();
     if (DYN && !a.dyn->active) return;  // the adaptive run has ended (uniform over the grid)
-    if (tid == 0) {
+    if (threadIdx.x == 0 && threadIdx.y == 0) {
       const int r0 = k0 / n2;
       const int r1 = (min(k0 + KT, nk) - 1) / n2;
       const uint32_t hbytes = (uint32_t)((r1 - r0 + 1) * 2 * nc * NT * sizeof(double2));
@@ -131,10 +130,38 @@ __global__ void __launch_bounds__(KT* TriEP<N>::NT, RowsEP<N, KT>::BLOCKS) k_rhs
     for (int x = 0; x < 3; x++)
       if ((a.dmask >> x) & 1) De[x] = tb.D[(size_t)(x * NT + e) * nk + k];
   }
-  if (staged) {
-    __syncthreads();  // trig table + barrier init visible to all threads
-    mbar_wait(&bar, 0, tb.err);
+  // sum_b (w_b E_pump . b) rho_e(k + b): kGather neighbours in flight at a time (an
+  // unrolled loop takes its remainder one by one), the factors of the block formed
+  // once and not by every thread. 96 x 96, 8 bands, 4 vectors: 14.0 us a stage, 15.3 with
+  // the loop; 120 x 120 three-band Coulomb, 10 vectors: a third of the kernel before.
+  constexpr int kGather = FULL ? 4 : 6;
+  const int nsel = e_non0 ? a.nsel : 0;
+  double2 pn[kGather];
+  auto gather = [&](int c0) {
+#pragma unroll
+    for (int u = 0; u < kGather; u++)
+      if (c0 + u < nsel) pn[u] = a.src[(size_t)e * nk + tb.nbr[(size_t)a.sel[c0 + u] * nk + k]];
+  };
+  if (valid) gather(0);
+  const int tid = threadIdx.y * KT + threadIdx.x;
+  for (int c = tid; c < nsel; c += KT * NT) {
+    const int b = a.sel[c];
+#pragma unroll
+    for (int x = 0; x < 3; x++) sF[c][x] = cst->wb[b] * ef0[x] * cst->bvec[b][x];
   }
+  if (staged || nsel) __syncthreads();  // factors, trig table and barrier init visible to all threads
+  if (valid)
+    for (int c0 = 0; c0 < nsel; c0 += kGather) {
+      if (c0) gather(c0);
+#pragma unroll
+      for (int u = 0; u < kGather; u++)
+        if (c0 + u < nsel) {
+          G = cadd(G, cscale(pn[u], sF[c0 + u][0]));
+          G = cadd(G, cscale(pn[u], sF[c0 + u][1]));
+          G = cadd(G, cscale(pn[u], sF[c0 + u][2]));
+        }
+    }
+  if (staged) mbar_wait(&bar, 0, tb.err);
   if (valid) {
     if (tb.h && a.xw) {
       // diagonal basis: the term of k_coulomb_xw (screened, rotated back)
@@ -194,21 +221,6 @@ __global__ void __launch_bounds__(KT* TriEP<N>::NT, RowsEP<N, KT>::BLOCKS) k_rhs
         He = cadd(He, X);
       }
       if (a.hr_out) a.hr_out[(size_t)e * nk + k] = He;
-    }
-    if (e_non0) {
-      // sum_b (w_b E_pump . b) rho_e(k + b)
-#pragma unroll 6
-      for (int c = 0; c < a.nsel; c++) {
-        const int b = a.sel[c];
-        const int kb = tb.nbr[(size_t)b * nk + k];
-        const double2 pn = a.src[(size_t)e * nk + kb];
-        const double f0 = cst->wb[b] * ef0[0] * cst->bvec[b][0];
-        const double f1 = cst->wb[b] * ef0[1] * cst->bvec[b][1];
-        const double f2 = cst->wb[b] * ef0[2] * cst->bvec[b][2];
-        G = cadd(G, cscale(pn, f0));
-        G = cadd(G, cscale(pn, f1));
-        G = cadd(G, cscale(pn, f2));
-      }
     }
   }
   {
@@ -370,7 +382,7 @@ static cudaError_t launch_ep(const DevTables& tb, const DevConsts* cst, const St
     // rows of the k grid one block of KT consecutive k points can touch
     const int rows = (tb.n2 + KT - 2) / tb.n2 + 1;
     const size_t bytes = sizeof(double2) * ((size_t)rows * 2 * tb.ncut * NT + tb.ncut * KT);
-    const size_t static_bytes = RowsEP<N, KT>::FULL ? sizeof(double2) * 2 * RowsEP<N, KT>::SIZE + 1024 : sizeof(double2) * 3 * NT * KT;
+    const size_t static_bytes = RowsEP<N, KT>::FULL ? sizeof(double2) * 2 * RowsEP<N, KT>::SIZE + 2560 : sizeof(double2) * 3 * NT * KT + 1600;
     if (bytes + static_bytes <= 48 * 1024) {
       b.stage_rows = rows;
       dyn = bytes;
