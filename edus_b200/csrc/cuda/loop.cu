@@ -15,7 +15,7 @@
 // stencil gathers 0.4, the element's own work 0.8.
 //   60 x 60 hBN, RK4, a record every step: 14.8 us a step, 28.7 before
 //   24 x 24 hBN, RK4 (one cluster): 8.5 us a step, 13.8 before
-//   70 x 70 with core-hole decay, AB5: 5.8 us a step, 10.5 before
+//   70 x 70 with core-hole decay, AB5: 5.5 us a step, 10.5 before
 //
 // The blocks wait on one another, so the launch is cooperative (all blocks
 // resident) or one cluster; a wait is bounded and records kErrTimeout. Data
@@ -276,6 +276,14 @@ __global__ void __launch_bounds__(MAXT) k_loop(const __grid_constant__ LoopArgs 
     }
   };
   auto fetched = [&]() { asm volatile("cp.async.wait_all;" ::: "memory"); };
+  // relaxation pairs and rates: in global memory they were two dependent reads a
+  // pair past an L1 that every grid barrier empties, 1800 cycles a stage
+  __shared__ int sRel[N * N];
+  __shared__ double sRelT[N * N];
+  for (int t = tid; t < tb.n_diss; t += nthr) {
+    sRel[t] = a.cst->diss_i[t] * N + a.cst->diss_j[t];
+    sRelT[t] = a.cst->T[sRel[t]];
+  }
   fetch(0);
   fetched();
   __syncthreads();
@@ -486,8 +494,8 @@ __global__ void __launch_bounds__(MAXT) k_loop(const __grid_constant__ LoopArgs 
           // M = conj(U) P U^T is formed once per k point (k_rhs_ep's threads each form
           // every M they use)
           for (int t = 0; t < tb.n_diss; t++) {
-            const int ii = a.cst->diss_i[t], jj = a.cst->diss_j[t];
-            const double2 f = cscale(cmulc(cconj(S.sU[(jj * N + j) * KS + kl]), S.sU[(i * N + ii) * KS + kl]), a.cst->T[ii * N + jj]);
+            const int ii = sRel[t] / N, jj = sRel[t] % N;
+            const double2 f = cscale(cmulc(cconj(S.sU[(jj * N + j) * KS + kl]), S.sU[(i * N + ii) * KS + kl]), sRelT[t]);
             v = csub(v, cmul(f, S.sM[(ii * N + jj) * KS + kl]));
           }
           v = cadd(v, tii);
