@@ -1001,7 +1001,6 @@ int loop_prepare(edus_ctx* c) {
   a.res = c->res;
   a.nstartup = ab && P.p.ab_rk4_startup ? c->order - 1 : 0;
   a.kt = p.kt;
-  a.cluster = p.cluster;
   a.P1 = c->d_P1;
   a.Pb = c->d_Pb;
   a.ring = c->d_ring;

@@ -14,7 +14,7 @@
 // atomic and a poll through L2; an array of flags polled by every block took 2.4),
 // stencil gathers 0.4, the element's own work 0.8.
 //   60 x 60 hBN, RK4, a record every step: 14.8 us a step, 28.7 before
-//   24 x 24 hBN, RK4 (one cluster): 8.5 us a step, 13.8 before
+//   24 x 24 hBN, RK4 (one cluster): 6.7 us a step, 13.8 before
 //   70 x 70 with core-hole decay, AB5: 5.5 us a step, 10.5 before
 //
 // The blocks wait on one another, so the launch is cooperative (all blocks
@@ -65,8 +65,9 @@ struct LoopSmem {
   double *sPop, *sGc;
   int* sN;
   LoopStep* sS;
+  double2* sX;  // cluster: stage inputs that the other blocks read, [2][NT][KS]
   size_t bytes;
-  __host__ __device__ LoopSmem(unsigned char* base, const DevTables& tb, int nb, int ngc, int ncomp) {
+  __host__ __device__ LoopSmem(unsigned char* base, const DevTables& tb, int nb, int ngc, int ncomp, bool cluster) {
     size_t off = 0;
     auto take = [&](size_t b) {
       unsigned char* r = base + off;
@@ -82,12 +83,22 @@ struct LoopSmem {
     sGc = (double*)take(sizeof(double) * 2 * ngc);
     sN = (int*)take(sizeof(int) * nb * KS);
     sS = (LoopStep*)take(2 * sizeof(LoopStep));
+    sX = (double2*)take(cluster ? sizeof(double2) * 2 * NT * KS : 0);
     bytes = off;
   }
 };
 
 __device__ __forceinline__ void cp_async16(void* dst, const void* src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+}
+
+// Entry off (in double2) of block rank's copy of the shared array at base.
+__device__ __forceinline__ double2 ld_cluster(uint32_t base, int rank, int off) {
+  uint32_t at;
+  double2 v;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"(base), "r"(rank));
+  asm volatile("ld.shared::cluster.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "r"(at + 16u * (uint32_t)off) : "memory");
+  return v;
 }
 
 // Barrier over all blocks; false when the bounded wait ran out (the same for
@@ -146,21 +157,26 @@ __device__ __forceinline__ double warp_sums(double (&v)[M]) {
   return x;
 }
 
-template <int N, bool AB, int MAXT>
+// CL: one cluster, the stage inputs exchanged through distributed shared memory
+// and written to global memory in the last step only. The barrier's release has
+// then no global stores to wait for (0.28 us for 0.9) and a gather is a read
+// of another SM's shared memory, not of L2. 24 x 24 hBN, RK4: 6.7 us a step, 8.0
+// with the exchange through L2.
+template <int N, bool AB, int MAXT, bool CL>
 __global__ void __launch_bounds__(MAXT) k_loop(const __grid_constant__ LoopArgs a) {
   constexpr int NT = TriL<N>::NT, KS = MAXT / NT;
   const DevTables& tb = a.tb;
   extern __shared__ __align__(16) unsigned char loop_smem_raw[];
   const int kt = a.kt, nk = tb.nk, nb = a.nb_sel, npc = a.npc, nbp = a.nbp, ngc = a.ngc;
   const int ncomp = a.ncomp;
-  const LoopSmem<N, MAXT> S(loop_smem_raw, tb, nb, ngc, ncomp);
+  const LoopSmem<N, MAXT> S(loop_smem_raw, tb, nb, ngc, ncomp, CL);
   __shared__ double sW[MAXT / 32][33];
   __shared__ double sT[kFields];
   __shared__ bool sOk;
   const int tid = threadIdx.x, nthr = blockDim.x, lane = tid % 32, warp = tid / 32, nwarp = nthr / 32;
   const int nstep_blocks = gridDim.x - 1;
   const bool stepper = (int)blockIdx.x < nstep_blocks;
-  GridBar bar{a.bar, 0u, gridDim.x, tb.err, a.cluster != 0, &sOk};
+  GridBar bar{a.bar, 0u, gridDim.x, tb.err, CL, &sOk};
 
   // ---------------------------------------------------------- the adding block
   // Joins every barrier; after the first one behind an instant the partials are
@@ -170,6 +186,7 @@ __global__ void __launch_bounds__(MAXT) k_loop(const __grid_constant__ LoopArgs 
     constexpr int kF = kSumF + N + 2;  // fields of a partial: currents, populations, max, min
     static_assert(kF <= 32, "a partial is one 32-word row");
     int inst = 0;
+    if (CL) bar.sync();  // the first stage inputs
     for (int it = 0; it < a.nsteps; it++) {
       const bool obs = (a.it0 + it) % a.res == 0;
       const int nbar = AB && a.it0 + it >= a.nstartup ? 1 : 4;
@@ -265,7 +282,12 @@ __global__ void __launch_bounds__(MAXT) k_loop(const __grid_constant__ LoopArgs 
   if (tb.n_diss > 0)
     for (int t = tid; t < N * N * kt; t += nthr) S.sU[(t / kt) * KS + t % kt] = tb.U[(size_t)(t / kt) * nk + min((int)(blockIdx.x * kt) + t % kt, nk - 1)];
   for (int t = tid; t < nb * kt; t += nthr)
-    S.sN[(t / kt) * KS + t % kt] = tb.nbr[(size_t)a.bsel[t / kt] * nk + min((int)(blockIdx.x * kt) + t % kt, nk - 1)];
+  {
+    const int kb = tb.nbr[(size_t)a.bsel[t / kt] * nk + min((int)(blockIdx.x * kt) + t % kt, nk - 1)];
+    S.sN[(t / kt) * KS + t % kt] = CL ? (kb / kt) << 16 | kb % kt : kb;  // CL: block and place
+  }
+  const uint32_t xbase = smem_u32(S.sX);
+  if (CL && valid) S.sX[e * KS + kl] = Pe;
   // step record it and its gradient coefficients into buffer it & 1, asynchronously
   auto fetch = [&](int it) {
     if (it < a.nsteps) {
@@ -286,11 +308,20 @@ __global__ void __launch_bounds__(MAXT) k_loop(const __grid_constant__ LoopArgs 
   }
   fetch(0);
   fetched();
-  __syncthreads();
+  if (CL)
+    bar.sync();
+  else
+    __syncthreads();
   double2 tii = cz();  // relaxation towards the filled bands: constant
   if (tb.n_diss > 0 && valid)
     for (int q = 0; q < tb.nbands; q++)
       tii = cadd(tii, cscale(cmulc(S.sU[(q * N + i) * KS + kl], S.sU[(q * N + j) * KS + kl]), a.cst->T[q * N + q]));
+  // stage input kb of this element: from L2, or from the block that owns it
+  int xb = 0;  // CL: half of sX with the stage inputs
+  auto input = [&](const double2* src, int kb) {
+    if constexpr (CL) return ld_cluster(xbase, kb >> 16, (xb * NT + e) * KS + (kb & 0xFFFF));
+    else return __ldcg(src + (size_t)e * nk + kb);
+  };
   double2* cur = a.P0;   // buffer of the current state
   double2* oth = a.Pa;
   int inst = 0;
@@ -437,6 +468,12 @@ __global__ void __launch_bounds__(MAXT) k_loop(const __grid_constant__ LoopArgs 
     const int nstage = rk ? 4 : 1;
     double2 pin = Pe;
     const double2* src = cur;
+    const bool last = it == a.nsteps - 1;
+    // the next stage's input, read by the other blocks behind the barrier
+    auto hand = [&](double2* dst, double2 x) {
+      if (CL) S.sX[((xb ^ 1) * NT + e) * KS + kl] = x;
+      if (!CL || last) dst[o] = x;
+    };
     for (int sg = 0; sg < nstage; sg++) {
       const int fi = sg == 0 ? 0 : (sg == 3 ? 2 : 1);
       // stencil gathers in flight before the element's own work
@@ -444,7 +481,7 @@ __global__ void __launch_bounds__(MAXT) k_loop(const __grid_constant__ LoopArgs 
       double2 pn[NG];
       const bool grad = st.e_non0 && valid;
 #pragma unroll
-      for (int c = 0; c < NG; c++) pn[c] = grad && c < nb ? __ldcg(src + (size_t)e * nk + S.sN[c * KS + kl]) : cz();
+      for (int c = 0; c < NG; c++) pn[c] = grad && c < nb ? input(src, S.sN[c * KS + kl]) : cz();
       if (own) {
         const int w = (i < tb.nch) != (j < tb.nch);
         double2 hu = He, hl = cconj(He);
@@ -517,7 +554,7 @@ __global__ void __launch_bounds__(MAXT) k_loop(const __grid_constant__ LoopArgs 
           for (int c0 = NG; c0 < nb; c0 += 6) {
             double2 p[6];
 #pragma unroll
-            for (int c = 0; c < 6; c++) p[c] = c0 + c < nb ? __ldcg(src + (size_t)e * nk + S.sN[(c0 + c) * KS + kl]) : cz();
+            for (int c = 0; c < 6; c++) p[c] = c0 + c < nb ? input(src, S.sN[(c0 + c) * KS + kl]) : cz();
             add(p, c0, std::integral_constant<int, 6>());
           }
         }
@@ -532,15 +569,15 @@ __global__ void __launch_bounds__(MAXT) k_loop(const __grid_constant__ LoopArgs 
             }
             acc = cadd(Pe, cscale(v, a.dt6));
             pin = cadd(Pe, cscale(v, a.dt2));
-            oth[o] = pin;
+            hand(oth, pin);
           } else if (sg < 3) {
             acc = cadd(acc, cscale(v, a.dt3));
             pin = cadd(Pe, cscale(v, sg == 1 ? a.dt2 : a.dt));
-            (sg == 1 ? a.Pb : oth)[o] = pin;
-            if (sg == 2 && (AB || it == a.nsteps - 1)) a.P1[o] = acc;
+            hand(sg == 1 ? a.Pb : oth, pin);
+            if (sg == 2 && (AB || last)) a.P1[o] = acc;
           } else {
             Pe = cadd(acc, cscale(v, a.dt6));
-            cur[o] = Pe;
+            hand(cur, Pe);
           }
         } else if (AB) {
           double2 d = cz();
@@ -552,9 +589,10 @@ __global__ void __launch_bounds__(MAXT) k_loop(const __grid_constant__ LoopArgs 
           for (int q = 3; q > 0; q--) R[AB ? q : 0] = R[AB ? q - 1 : 0];
           R[0] = v;
           Pe = cadd(Pe, cscale(d, a.dt));
-          oth[o] = Pe;
+          hand(oth, Pe);
         }
       }
+      xb ^= 1;
       if (rk) src = sg == 1 ? a.Pb : oth;
       if (sg == nstage - 1) fetched();
       if (!bar.sync()) return;
@@ -572,11 +610,11 @@ __global__ void __launch_bounds__(MAXT) k_loop(const __grid_constant__ LoopArgs 
   }
 }
 
-template <int N, bool AB, int MAXT>
+template <int N, bool AB, int MAXT, bool CL>
 cudaError_t loop_launch_t(const LoopArgs& a, const LoopPlan& p, cudaStream_t s) {
-  cudaError_t e = cudaFuncSetAttribute(k_loop<N, AB, MAXT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem);
-  if (e == cudaSuccess && p.cluster && p.blocks + 1 > 8)
-    e = cudaFuncSetAttribute(k_loop<N, AB, MAXT>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  cudaError_t e = cudaFuncSetAttribute(k_loop<N, AB, MAXT, CL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem);
+  if (e == cudaSuccess && CL && p.blocks + 1 > 8)
+    e = cudaFuncSetAttribute(k_loop<N, AB, MAXT, CL>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
   if (e != cudaSuccess) return e;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(p.blocks + 1);
@@ -584,7 +622,7 @@ cudaError_t loop_launch_t(const LoopArgs& a, const LoopPlan& p, cudaStream_t s) 
   cfg.dynamicSmemBytes = p.smem;
   cfg.stream = s;
   cudaLaunchAttribute at[1];
-  if (p.cluster) {
+  if (CL) {
     at[0].id = cudaLaunchAttributeClusterDimension;
     at[0].val.clusterDim.x = p.blocks + 1;
     at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
@@ -594,17 +632,19 @@ cudaError_t loop_launch_t(const LoopArgs& a, const LoopPlan& p, cudaStream_t s) 
   }
   cfg.attrs = at;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, k_loop<N, AB, MAXT>, a);
+  return cudaLaunchKernelEx(&cfg, k_loop<N, AB, MAXT, CL>, a);
 }
 
 template <int N, bool AB>
 cudaError_t loop_launch(const LoopArgs& a, const LoopPlan& p, cudaStream_t s) {
-  return p.small ? loop_launch_t<N, AB, kLoopSmall>(a, p, s) : loop_launch_t<N, AB, kLoopThreads>(a, p, s);
+  if (p.cluster) return p.small ? loop_launch_t<N, AB, kLoopSmall, true>(a, p, s) : cudaErrorInvalidValue;
+  return p.small ? loop_launch_t<N, AB, kLoopSmall, false>(a, p, s) : loop_launch_t<N, AB, kLoopThreads, false>(a, p, s);
 }
 
 template <int N>
-size_t loop_smem(const DevTables& tb, bool small, int nb, int ngc, int ncomp) {
-  return small ? LoopSmem<N, kLoopSmall>(nullptr, tb, nb, ngc, ncomp).bytes : LoopSmem<N, kLoopThreads>(nullptr, tb, nb, ngc, ncomp).bytes;
+size_t loop_smem(const DevTables& tb, bool small, int nb, int ngc, int ncomp, bool cluster) {
+  return small ? LoopSmem<N, kLoopSmall>(nullptr, tb, nb, ngc, ncomp, cluster).bytes
+               : LoopSmem<N, kLoopThreads>(nullptr, tb, nb, ngc, ncomp, cluster).bytes;
 }
 
 }  // namespace
@@ -629,11 +669,11 @@ LoopPlan loop_plan(const DevTables& tb, int nb, int ngc, int ncomp, int sms) {
   if (threads > kLoopThreads || p.kt > kLoopThreads / nt || blocks < 1) return p;
   p.small = threads <= kLoopSmall && p.kt <= kLoopSmall / nt;
   switch (tb.n) {
-    case 1: p.smem = loop_smem<1>(tb, p.small, nb, ngc, ncomp); break;
-    case 2: p.smem = loop_smem<2>(tb, p.small, nb, ngc, ncomp); break;
-    case 3: p.smem = loop_smem<3>(tb, p.small, nb, ngc, ncomp); break;
-    case 4: p.smem = loop_smem<4>(tb, p.small, nb, ngc, ncomp); break;
-    case 5: p.smem = loop_smem<5>(tb, p.small, nb, ngc, ncomp); break;
+    case 1: p.smem = loop_smem<1>(tb, p.small, nb, ngc, ncomp, p.cluster); break;
+    case 2: p.smem = loop_smem<2>(tb, p.small, nb, ngc, ncomp, p.cluster); break;
+    case 3: p.smem = loop_smem<3>(tb, p.small, nb, ngc, ncomp, p.cluster); break;
+    case 4: p.smem = loop_smem<4>(tb, p.small, nb, ngc, ncomp, p.cluster); break;
+    case 5: p.smem = loop_smem<5>(tb, p.small, nb, ngc, ncomp, p.cluster); break;
   }
   if (p.smem > 220 * 1024) return p;
   p.threads = threads;

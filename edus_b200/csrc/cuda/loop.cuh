@@ -27,7 +27,6 @@ struct LoopArgs {
   size_t stride;               // bytes per step, a multiple of 16
   int it0, res, nstartup;  // first step, output resolution, RK4 steps of the Adams-Bashforth start-up
   int nsteps, order, kt;   // order 0: RK4; kt: k points per block
-  int cluster;             // 1: the grid is one cluster
   double2 *P0, *P1, *Pa, *Pb;
   double2* ring;           // Adams-Bashforth: derivatives before the first step, newest first, and after the last
   double dt, dt6, dt3, dt2, wx2;

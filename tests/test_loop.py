@@ -60,6 +60,13 @@ def test_one_launch_matches_launch_per_stage(workdir, kind, n1, n2, solver, one)
         b.reset()
 
 
+# stage inputs through distributed shared memory (one cluster): one block, two, a last block
+# that is partly filled, all 15
+@pytest.mark.parametrize("kind,n1,n2,solver", [("hbn", 4, 4, AB4), ("hbn", 6, 6, ""), ("hbn", 18, 22, AB4), ("hbn", 30, 32, AB4), (2, 24, 26, ""), (5, 18, 20, AB4)])
+def test_one_cluster_matches_launch_per_stage(workdir, kind, n1, n2, solver):
+    test_one_launch_matches_launch_per_stage(workdir, kind, n1, n2, solver, True)
+
+
 def test_run_of_several_launches_keeps_the_history(workdir):
     """More steps than one launch takes: Adams-Bashforth's derivatives cross the gap."""
     pb = make(workdir, "hbn", 8, 8, "Adams_Bashforth 5\n", 500, t_fin=170.0)
