@@ -230,6 +230,7 @@ int state_to_dev(edus_ctx* c, const double* rho, double2* d) {
 int state_from_dev(edus_ctx* c, const double2* d, double* rho) {
   const int n = c->n, nk = c->nk;
   const size_t bytes = sizeof(double2) * (size_t)n * n * nk;
+  CK(cudaSetDevice(c->device));
   if (!c->d_full && dalloc(c, &c->d_full, (size_t)n * n * nk)) {
     clear_error();
     cudaGetLastError();
