@@ -46,25 +46,34 @@ struct TriEP {
 // Exchange rows of the full-matrix form (8 and 16 bands): entry (r, c) of k point
 // kl at [r * RS + c * KT + kl]; the padded row stride puts the rows that the
 // elements (i, j), (i, j + 1), ... of a warp read on different banks.
-template <int N, int KT>
+template <int N, int KT, bool DYN>
 struct RowsEP {
   static constexpr bool FULL = N >= 8;
   static constexpr int RS = N * KT + KT, SIZE = FULL ? N * RS : 1;
-  // Resident blocks the registers are sized for. 8 bands: three blocks of 288
-  // threads (8 k points; 62.3 us a step on 96 x 96), against 73.8 for two of 576 and
-  // 73.5 for four of 288, which spill, and 87.6 for one of 576 as the element-parallel
-  // form ran. 16 bands: one block of 544 (51.3 us on 30 x 34; two 53.8, three 68.6).
-  // 3 bands: four blocks of 192 (80 registers, no spills), so that 120 x 120 k points,
-  // 450 blocks, are one wave and not two of 296.
-  static constexpr int BLOCKS = N == 8 ? 3 : (N == 3 ? 4 : 1);
+  // Resident blocks the registers are sized for; 0 leaves them to the compiler, where
+  // naming one block would let it take all (110 registers for 2 bands, 132 for 4).
+  // 8 bands: three blocks of 288 threads (8 k points; 62.3 us a step on 96 x 96), against
+  // 73.8 for two of 576, 73.5 for four of 288 and 87.6 for one of 576 as the
+  // element-parallel form ran. 16 bands: one block of 544 (51.3 us on 30 x 34; two 53.8,
+  // three 68.6). Both spill (100 and 148 bytes). 2 bands: seven of 96 (80 registers; 192 x 192, 14
+  // vectors, RK4: 20.0 us a step, 32.5 with 110 registers). 3 bands:
+  // four of 192 (80 registers): 120 x 120 k points, 450 blocks, are one wave. 4 bands:
+  // two of 320 (96 registers; 112 x 112: 29.8 us a step, 37.9 with one).
+  static constexpr int BLOCKS = N == 8 ? 3 : (N == 16 ? 1 : (N == 2 ? 7 : (DYN ? 0 : (N == 3 ? 4 : (N == 4 ? 2 : 0)))));
+  // Stencil neighbours in flight at a time, and whether the adaptive step's scalars are
+  // read where they are used and not before: what fits the registers above. Adaptive
+  // step, 3 bands: 27.8 us a step on 60 x 60 and 31.8 on 120 x 120 (31.2 and 35.5 with six
+  // neighbours and early scalars, which spill 96 bytes).
+  static constexpr int GATHER = FULL ? 4 : (DYN ? (N <= 2 ? 6 : (N == 3 ? 5 : 4)) : (N == 2 ? 5 : 6));
+  static constexpr bool LATE = DYN && N == 3;
 };
 
 // DYN: the stage scalars come from the adaptive step's device copy (a.dyn);
 // a separate instantiation so the constant-step kernel keeps its registers.
 template <int N, int KT, bool DYN>
-__global__ void __launch_bounds__(KT* TriEP<N>::NT, RowsEP<N, KT>::BLOCKS) k_rhs_ep(DevTables tb, const DevConsts* __restrict__ cst, StageArgs a) {
+__global__ void __launch_bounds__(KT* TriEP<N>::NT, RowsEP<N, KT, DYN>::BLOCKS) k_rhs_ep(DevTables tb, const DevConsts* __restrict__ cst, StageArgs a) {
   constexpr int NT = TriEP<N>::NT;
-  using Rows = RowsEP<N, KT>;
+  using Rows = RowsEP<N, KT, DYN>;
   constexpr bool FULL = Rows::FULL;
   constexpr int RS = Rows::RS;
   __shared__ double2 sP[FULL ? 1 : NT][KT];
@@ -117,10 +126,14 @@ __global__ void __launch_bounds__(KT* TriEP<N>::NT, RowsEP<N, KT>::BLOCKS) k_rhs
     ef1[x] = dy ? dy->EF[a.dyn_field][1][x] : a.EF[1][x];
   }
   const int e_non0 = dy ? dy->e_non0 : a.e_non0;
-  const double c1 = dy ? dy->c[a.dyn_stage][0] : a.c1;
-  const double c2 = dy ? dy->c[a.dyn_stage][1] : a.c2;
-  const double dtv = dy ? dy->dt : a.dt;
-  const double pcn = dy ? (*dy->pcmax + *dy->ncond) : a.pcond_plus_ncond;
+  double c1, c2, dtv, pcn;
+  auto step_scalars = [&]() {
+    c1 = dy ? dy->c[a.dyn_stage][0] : a.c1;
+    c2 = dy ? dy->c[a.dyn_stage][1] : a.c2;
+    dtv = dy ? dy->dt : a.dt;
+    pcn = dy ? (*dy->pcmax + *dy->ncond) : a.pcond_plus_ncond;
+  };
+  if (!Rows::LATE) step_scalars();
   double2 Pe = cz(), He = cz(), G = cz();
   double2 De[3] = {cz(), cz(), cz()};
   if (valid) {
@@ -133,8 +146,11 @@ __global__ void __launch_bounds__(KT* TriEP<N>::NT, RowsEP<N, KT>::BLOCKS) k_rhs
   // sum_b (w_b E_pump . b) rho_e(k + b): kGather neighbours in flight at a time (an
   // unrolled loop takes its remainder one by one), the factors of the block formed
   // once and not by every thread. 96 x 96, 8 bands, 4 vectors: 14.0 us a stage, 15.3 with
-  // the loop; 120 x 120 three-band Coulomb, 10 vectors: a third of the kernel before.
-  constexpr int kGather = FULL ? 4 : 6;
+  // the loop. Up to 5 bands the first two groups stand by themselves: their entries of a.sel
+  // are then at constant places, while an index that is not constant costs a
+  // dependent read a vector (3 bands, 144 x 144, RK4: 28.3 us a step, 29.9 in the loop; 4 bands,
+  // 108 x 108: 34.0, 36.4).
+  constexpr int kGather = Rows::GATHER;
   const int nsel = e_non0 ? a.nsel : 0;
   double2 pn[kGather];
   auto gather = [&](int c0) {
@@ -150,17 +166,33 @@ __global__ void __launch_bounds__(KT* TriEP<N>::NT, RowsEP<N, KT>::BLOCKS) k_rhs
     for (int x = 0; x < 3; x++) sF[c][x] = cst->wb[b] * ef0[x] * cst->bvec[b][x];
   }
   if (staged || nsel) __syncthreads();  // factors, trig table and barrier init visible to all threads
-  if (valid)
-    for (int c0 = 0; c0 < nsel; c0 += kGather) {
-      if (c0) gather(c0);
+  auto add = [&](int c0) {
 #pragma unroll
-      for (int u = 0; u < kGather; u++)
-        if (c0 + u < nsel) {
-          G = cadd(G, cscale(pn[u], sF[c0 + u][0]));
-          G = cadd(G, cscale(pn[u], sF[c0 + u][1]));
-          G = cadd(G, cscale(pn[u], sF[c0 + u][2]));
+    for (int u = 0; u < kGather; u++)
+      if (c0 + u < nsel) {
+        G = cadd(G, cscale(pn[u], sF[c0 + u][0]));
+        G = cadd(G, cscale(pn[u], sF[c0 + u][1]));
+        G = cadd(G, cscale(pn[u], sF[c0 + u][2]));
+      }
+  };
+  if (valid && nsel) {
+    if constexpr (FULL) {
+      for (int c0 = 0; c0 < nsel; c0 += kGather) {
+        if (c0) gather(c0);
+        add(c0);
+      }
+    } else {
+      add(0);
+      if (nsel > kGather) {
+        gather(kGather);
+        add(kGather);
+        for (int c0 = 2 * kGather; c0 < nsel; c0 += kGather) {
+          gather(c0);
+          add(c0);
         }
+      }
     }
+  }
   if (staged) mbar_wait(&bar, 0, tb.err);
   if (valid) {
     if (tb.h && a.xw) {
@@ -248,6 +280,7 @@ __global__ void __launch_bounds__(KT* TriEP<N>::NT, RowsEP<N, KT>::BLOCKS) k_rhs
     }
   }
   __syncthreads();
+  if (Rows::LATE) step_scalars();
 
   double dpmax = 0.;
   if (valid) {
@@ -382,7 +415,7 @@ static cudaError_t launch_ep(const DevTables& tb, const DevConsts* cst, const St
     // rows of the k grid one block of KT consecutive k points can touch
     const int rows = (tb.n2 + KT - 2) / tb.n2 + 1;
     const size_t bytes = sizeof(double2) * ((size_t)rows * 2 * tb.ncut * NT + tb.ncut * KT);
-    const size_t static_bytes = RowsEP<N, KT>::FULL ? sizeof(double2) * 2 * RowsEP<N, KT>::SIZE + 2560 : sizeof(double2) * 3 * NT * KT + 1600;
+    const size_t static_bytes = RowsEP<N, KT, false>::FULL ? sizeof(double2) * 2 * RowsEP<N, KT, false>::SIZE + 2560 : sizeof(double2) * 3 * NT * KT + 1600;
     if (bytes + static_bytes <= 48 * 1024) {
       b.stage_rows = rows;
       dyn = bytes;
