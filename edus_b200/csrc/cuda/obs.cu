@@ -78,9 +78,9 @@ static_assert(kFields * sizeof(double) <= sizeof(ObsPart), "partials are sized b
 // blocks of k_obs_el: enough for three 256- or two 512-thread blocks on every SM
 constexpr int kObsElBlocks = 512;
 
-// The output record from the totals T of every field (one thread).
-template <int N>
-__device__ __forceinline__ void obs_record(const DevTables& tb, const ObsArgs& a, const double* T) {
+// The output record from the totals T(f) of every field (one thread).
+template <int N, class F>
+__device__ __forceinline__ void obs_record(const DevTables& tb, const ObsArgs& a, const F& T) {
   ObsRecord rec = a.rec;
   ObsRecord* slot = a.log;
   if (a.dyn) {
@@ -96,7 +96,7 @@ __device__ __forceinline__ void obs_record(const DevTables& tb, const ObsArgs& a
   const double nc = obs_fill(rec, T, N, tb.nk, tb.nbands, a.scaleJ, a.scaleTA);
   if (slot) *slot = rec;
   if (a.ncond_dev) *a.ncond_dev = nc;
-  if (a.pcmax_dev) *a.pcmax_dev = T[kFMax];
+  if (a.pcmax_dev) *a.pcmax_dev = T(kFMax);
   *a.done = 0u;
 }
 
@@ -128,7 +128,7 @@ __device__ __forceinline__ void obs_finish(const DevTables& tb, const ObsArgs& a
     if (lane == 0) T[f] = x;
   }
   __syncthreads();
-  if (threadIdx.x == 0) obs_record<N>(tb, a, T);
+  if (threadIdx.x == 0) obs_record<N>(tb, a, [&](int f) { return T[f]; });
 }
 
 // One thread per k point.
@@ -289,21 +289,13 @@ __global__ void __launch_bounds__(kObsThreads) k_obs(DevTables tb, const DevCons
   }
   if (threadIdx.x != 0) return;
   const ObsPart& S = sp[0];
-  double T[kFields];
-  for (int i = 0; i < N; i++) T[i] = S.pop[i];
-  for (int x = 0; x < 3; x++) {
-    double* f = T + kFX + kPerX * x;
-    f[0] = S.J1[x].x;
-    f[1] = S.J1[x].y;
-    f[2] = S.J2[x].y;
-    f[3] = S.TA[x].x;
-    f[4] = S.TA[x].y;
-    f[5] = S.PL[x].x;
-    f[6] = S.PL[x].y;
-  }
-  T[kFMax] = S.pmax;
-  T[kFMin] = S.pmin;
-  obs_record<N>(tb, a, T);
+  obs_record<N>(tb, a, [&](int f) {  // (f is a constant at every use)
+    if (f < kFX) return S.pop[f];
+    if (f >= kFMax) return f == kFMax ? S.pmax : S.pmin;
+    const int x = (f - kFX) / kPerX, m = (f - kFX) % kPerX;
+    const double2 z = m < 2 ? S.J1[x] : (m < 3 ? S.J2[x] : (m < 5 ? S.TA[x] : S.PL[x]));
+    return m == 0 || m == 3 || m == 5 ? z.x : z.y;
+  });
 }
 
 // One thread per (k point, entry (b, l) of the full matrices), KO k points at a

@@ -28,32 +28,33 @@ __device__ __forceinline__ double tree128(int f, double v0, double v1, double v2
 template <int N>
 __device__ __forceinline__ int field_no(int v) { return v < N ? v : kFX + (v - N); }
 
-// The record's sums from the totals T of every field; returns n_cond.
-__device__ __forceinline__ double obs_fill(ObsRecord& rec, const double* T, int n, int nk, int nbands, double scaleJ,
-                                           double scaleTA) {
+// The record's sums from the totals T(f) of every field; returns n_cond.
+template <class F>
+__device__ __forceinline__ double obs_fill(ObsRecord& rec, const F& T, int n, int nk, int nbands, double scaleJ, double scaleTA) {
   const double inv = 1. / nk;
   double trace = -(double)nbands;
   double nc = 0;
   for (int i = 0; i < n; i++) {
-    double v = T[i] * inv;
+    double v = T(i) * inv;
     trace += v;
     if (i < nbands) v = 1.0 - v;
     rec.pop[i] = v;
     if (v > nc) nc = v;
   }
+#pragma unroll
   for (int x = 0; x < 3; x++) {
-    const double* f = T + kFX + kPerX * x;
-    rec.J1[2 * x] = f[0] * scaleJ;
-    rec.J1[2 * x + 1] = f[1] * scaleJ;
-    rec.J2[x] = -2. * (f[2] * scaleJ);
-    rec.tabs[2 * x] = f[3] * scaleTA * inv;
-    rec.tabs[2 * x + 1] = f[4] * scaleTA * inv;
-    rec.pol[2 * x] = f[5] * inv;
-    rec.pol[2 * x + 1] = f[6] * inv;
+    const int f = kFX + kPerX * x;
+    rec.J1[2 * x] = T(f) * scaleJ;
+    rec.J1[2 * x + 1] = T(f + 1) * scaleJ;
+    rec.J2[x] = -2. * (T(f + 2) * scaleJ);
+    rec.tabs[2 * x] = T(f + 3) * scaleTA * inv;
+    rec.tabs[2 * x + 1] = T(f + 4) * scaleTA * inv;
+    rec.pol[2 * x] = T(f + 5) * inv;
+    rec.pol[2 * x + 1] = T(f + 6) * inv;
   }
   rec.trace_dev = trace;
-  rec.p_cond_max = T[kFMax];
-  rec.p_min = T[kFMin];
+  rec.p_cond_max = T(kFMax);
+  rec.p_min = T(kFMin);
   rec.n_cond = nc;
   return nc;
 }
