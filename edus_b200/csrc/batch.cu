@@ -20,6 +20,7 @@
 #include "cuda/kernels.hpp"
 #include "cuda/model_build.hpp"
 #include "cuda/tc_contract.hpp"
+#include "host/device_work.hpp"
 #include "host/problem.hpp"
 
 namespace edus {
@@ -1178,6 +1179,7 @@ int edus_batch_add(edus_batch* b, const edus_problem* pb, int64_t tag, int32_t* 
 int edus_batch_advance(edus_batch* b, int32_t nsteps) {
   if (!b || nsteps < 0) return fail(EDUS_EINVAL, "bad argument");
   BCK(cudaSetDevice(b->device));
+  const DeviceWork work(b->device);
   const int S = b->opt.chunk_steps;
   bool tiles = false;
   for (auto& kv : b->classes) tiles = tiles || !kv.second.tiles.empty();
@@ -1311,6 +1313,7 @@ int edus_batch_tile_k(edus_batch* b, int32_t nbands, int32_t* kt) {
 int edus_batch_profile(edus_batch* b, int32_t nsteps, edus_kernel_time* out, int32_t cap, int32_t* n) {
   if (!b || nsteps < 0 || !out || cap < 0 || !n) return fail(EDUS_EINVAL, "bad argument");
   BCK(cudaSetDevice(b->device));
+  const DeviceWork work(b->device);
   std::map<std::pair<int, int>, edus_kernel_time> acc;
   const int S = b->opt.chunk_steps;
   for (int done = 0; done < nsteps; done += S) {

@@ -17,6 +17,7 @@
 #include <fstream>
 #include <functional>
 #include <iomanip>
+#include <memory>
 #include <mutex>
 #include <sstream>
 #include <string>
@@ -28,6 +29,7 @@
 #include "cuda/tc_contract.hpp"
 #include "cuda/dyn.cuh"
 #include "cuda/loop.cuh"
+#include "host/device_work.hpp"
 #include "host/problem.hpp"
 
 namespace edus {
@@ -79,6 +81,7 @@ struct edus_ctx {
   edus_obs* d_obs_one = nullptr;  // record of edus_observables, allocated on its first call
   size_t dev_bytes = 0;            // device memory the context holds
   long long async_l0 = 0;          // launch count at the start of an asynchronous whole run
+  std::unique_ptr<DeviceWork> async_work;  // from its start to its end
   int log_cap = 0, nlog = 0;
   double* d_ncond = nullptr;
   double* d_pcmax = nullptr;
@@ -1065,9 +1068,10 @@ int loop_run(edus_ctx* c) {
 }
 
 // Enqueue nsteps (or the whole run) between the context's two timing events;
-// *l0 receives the launch count before them. timed_finish waits for the end
+// *l0 receives the launch count before them. alone: nothing else of the process
+// is at work on the device (device_work.hpp). timed_finish waits for the end
 // event and checks the device error word.
-int timed_start(edus_ctx* c, int nsteps, bool all, long long* l0_out, bool alone = true) {
+int timed_start(edus_ctx* c, int nsteps, bool all, long long* l0_out, bool alone) {
   CK(cudaSetDevice(c->device));
   long long l0 = c->launches;
   *l0_out = l0;
@@ -1079,8 +1083,8 @@ int timed_start(edus_ctx* c, int nsteps, bool all, long long* l0_out, bool alone
     return 0;
   }
   const bool graph = all && !c->dyn && c->use_graphs && c->it == 0;
-  // (a run that shares the GPU with a batch keeps the graph: its small kernels
-  // run beside the batch's, blocks that wait on one another would not)
+  // (a run that shares the GPU keeps the graph: its small kernels run beside the
+  // others', blocks that wait on one another would not)
   if (graph && alone && !c->profiling) {
     if (!c->loop_tried) {
       int rc = loop_prepare(c);
@@ -1168,8 +1172,9 @@ int timed_finish(edus_ctx* c, long long l0) {
 }
 
 int timed(edus_ctx* c, int nsteps, bool all) {
+  const DeviceWork work(c->device);
   long long l0 = 0;
-  int rc = timed_start(c, nsteps, all, &l0);
+  int rc = timed_start(c, nsteps, all, &l0, work.alone());
   if (rc) return rc;
   return timed_finish(c, l0);
 }
@@ -1223,7 +1228,10 @@ int ctx_start_async(edus_ctx* c) {
   if (!c) return fail(EDUS_EINVAL, "null argument");
   if (c->dyn || !c->use_graphs || c->it != 0)
     return fail(EDUS_EUNSUPPORTED, "an asynchronous whole run needs a fresh context at constant dt with graphs");
-  return timed_start(c, 0, true, &c->async_l0, false);
+  c->async_work = std::make_unique<DeviceWork>(c->device);
+  const int rc = timed_start(c, 0, true, &c->async_l0, false);
+  if (rc) c->async_work.reset();
+  return rc;
 }
 
 int ctx_poll(edus_ctx* c, bool* done) {
@@ -1236,13 +1244,16 @@ int ctx_poll(edus_ctx* c, bool* done) {
   }
   if (e != cudaSuccess) return fail(EDUS_ECUDA, "context run: %s", cudaGetErrorString(e));
   *done = true;
+  c->async_work.reset();
   return timed_finish(c, c->async_l0);
 }
 
 int ctx_wait(edus_ctx* c) {
   if (!c) return fail(EDUS_EINVAL, "null argument");
   CK(cudaSetDevice(c->device));
-  return timed_finish(c, c->async_l0);
+  const int rc = timed_finish(c, c->async_l0);
+  c->async_work.reset();
+  return rc;
 }
 
 size_t ctx_device_bytes(const edus_ctx* c) { return c ? c->dev_bytes : 0; }
@@ -2291,6 +2302,7 @@ int edus_profile_ex(edus_ctx* c, int32_t nsteps, int32_t reps, double* rhs_ms, i
                     int64_t* coul_launches) {
   if (!c || nsteps < 0 || reps < 1) return fail(EDUS_EINVAL, "bad argument");
   CK(cudaSetDevice(c->device));
+  const DeviceWork work(c->device);
   c->profiling = true;
   c->prof_reps = reps;
   c->prof_pairs.clear();

@@ -54,6 +54,10 @@ struct TriL {
 constexpr int kLoopSmall = 384, kLoopThreads = 640;
 constexpr int kSumF = 3 * kPerX;   // current fields of a block partial
 
+// Polls of a grid barrier before it gives up, tens of seconds: at a launch's first
+// barrier the last blocks may still wait for room that another program's kernels hold.
+constexpr int kGridWaitIters = 1 << 26;
+
 __host__ __device__ constexpr size_t pad16(size_t b) { return (b + 15) & ~(size_t)15; }
 
 // Dynamic shared memory of a block of at most MAXT threads. Planes over the
@@ -120,7 +124,7 @@ struct GridBar {
     if (threadIdx.x == 0) {
       asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(ctr) : "memory");
       bool got = false;
-      for (int it = 0; it < kBulkWaitIters; ++it) {
+      for (int it = 0; it < kGridWaitIters; ++it) {
         unsigned int v;
         asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(ctr) : "memory");
         if ((int)(v - target) >= 0) {

@@ -25,6 +25,7 @@
 #include <vector>
 
 #include "ctx_hooks.hpp"
+#include "host/device_work.hpp"
 #include "host/problem.hpp"
 
 namespace {
@@ -348,9 +349,11 @@ int retire(edus_server* s) {
 
 void loop_main(edus_server* s) {
   cudaSetDevice(s->opt.batch.device);
+  std::unique_ptr<edus::DeviceWork> work;  // held while requests run, between chunks too
   for (;;) {
     {
       std::unique_lock<std::mutex> lk(s->mu);
+      if (s->running.empty()) work.reset();
       s->cv_loop.wait_for(lk, std::chrono::milliseconds(2), [&] {
         return s->stop || !s->ready.empty() || !s->running.empty() || !s->started.empty();
       });
@@ -366,6 +369,7 @@ void loop_main(edus_server* s) {
       std::lock_guard<std::mutex> lk(s->mu);
       any = !s->running.empty();
     }
+    if (any && !work) work = std::make_unique<edus::DeviceWork>(s->opt.batch.device);
     // with tiles, one chunk; with Coulomb contexts only, a poll (no wait)
     if (!rc && any)
       rc = edus::batch_has_tiles(s->batch) ? edus_batch_advance(s->batch, s->opt.batch.chunk_steps)

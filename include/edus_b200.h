@@ -276,7 +276,12 @@ int edus_get_state(edus_ctx* ctx, double* rho);
  * including the output instants every it_resolution steps, which are
  * appended to the context's observable log. */
 int edus_step(edus_ctx* ctx, int32_t nsteps);
-/* Run the whole time loop (itfi+1 steps for constant dt). */
+/* Run the whole time loop (itfi+1 steps for constant dt). Contexts may run in
+ * several threads at once. A run that begins while no other call of the process
+ * (a run or step of a context, a batch that advances, a server with requests) is at
+ * work on the device may take its steps in one launch; the others take a captured
+ * launch per stage. The two add the observables' k sums in a different order: they
+ * agree to FP64 rounding. */
 int edus_run(edus_ctx* ctx);
 /* Clock of the loop: iteration index, time (a.u.), current dt. */
 int edus_clock(edus_ctx* ctx, int32_t* it, double* t, double* dt);

@@ -10,3 +10,52 @@ def test_state_is_read_from_a_device_that_is_not_the_current_one(workdir):
     a, b = E.Context(pb, device=1), E.Context(pb, device=0)  # device 0 is current now
     assert a.get_state().shape == (64, 3, 3) and b.get_state().shape == (64, 3, 3)
     """)
+
+
+def test_whole_run_in_one_launch_only_where_nothing_else_is_at_work(workdir):
+    """A context that begins while another call of the process works on the device
+    takes the captured launch per stage; alone again, or on another device, one launch."""
+    run_host(workdir, """
+    hbn = problem(W.hbn_rk4(d + "/a", n=24, t_fin_fs=0.2))
+    cou = problem(W.hbn_coulomb(d + "/c", n=12, t_fin_fs=0.1))
+    a, b, far = E.Context(hbn), E.Context(hbn), E.Context(hbn, device=1)
+
+    def run(c):
+        F.fake_clear()
+        g = F.fake_graph_launches()
+        c.reset()
+        c.run()
+        assert c.clock()[0] == hbn.info.nsteps
+        return launches("k_loop"), F.fake_graph_launches() - g
+
+    @C.CFUNCTYPE(None)
+    def others():  # in the first wait of a call
+        F.fake_on_wait(None)
+        seen.append((run(b), run(far)))
+
+    def during(call):
+        global seen
+        seen = []
+        F.fake_on_wait(others)
+        call()
+        assert len(seen) == 1
+        return seen[0]
+
+    shared = ((0, 1), (1, 0))
+    assert run(b) == (1, 0)
+    assert during(a.run) == shared          # a whole run
+    a.reset()
+    assert during(lambda: a.step(3)) == shared
+    batch = E.Batch()
+    batch.add(problem(W.hbn_rk4(d + "/b", n=12, t_fin_fs=0.2)))
+    assert during(lambda: batch.advance(16)) == shared
+    assert run(b) == (1, 0) and run(b) == (1, 0)
+    slot = batch.add(cou)                    # runs by itself until it is polled
+    assert run(b) == (0, 1)
+    batch.advance(16)
+    assert batch.poll(slot)[0] == abi.EDUS_INST_DONE
+    assert run(b) == (1, 0)
+    batch.add(cou)
+    batch.close()                            # released without being polled
+    assert run(b) == (1, 0)
+    """)

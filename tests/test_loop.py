@@ -3,10 +3,13 @@ the same problem, at the sizes where the split over blocks can go wrong: a
 block that is partly filled, one cluster and many blocks, the largest grids the
 form takes and the first it leaves to the launch per stage, every band count it
 is built for, several launches in a row."""
+import threading
+
 import numpy as np
 import pytest
 
 import edus_b200 as E
+from edus_b200 import abi
 from edus_b200 import workloads as W
 
 pytestmark = pytest.mark.gpu
@@ -77,3 +80,32 @@ def test_run_of_several_launches_keeps_the_history(workdir):
     b.run()
     assert np.abs(a.get_state() - b.get_state()).max() <= 1e-13
     assert len(a.obs()) == len(b.obs())
+
+
+def test_runs_that_share_the_device(workdir):
+    """Contexts in threads of their own beside a batch that advances: every run ends
+    with the state of a run by itself."""
+    pb = make(workdir, "hbn", 60, 60, "", 3)
+    alone = E.Context(pb)
+    alone.run()
+    want, failed = alone.get_state(), []
+
+    def runs(c):
+        try:
+            for _ in range(4):
+                c.reset()
+                c.run()
+                assert np.abs(c.get_state() - want).max() <= 1e-13
+        except Exception as e:  # noqa: BLE001 (reported below)
+            failed.append(e)
+
+    batch = E.Batch()
+    slot = batch.add(make(workdir + "/b", "hbn", 48, 48, "", 5, t_fin=1.0))
+    threads = [threading.Thread(target=runs, args=(c,)) for c in [E.Context(pb) for _ in range(3)]]
+    for t in threads:
+        t.start()
+    while batch.poll(slot)[0] == abi.EDUS_INST_RUNNING:
+        batch.advance(16)
+    for t in threads:
+        t.join()
+    assert not failed, failed
