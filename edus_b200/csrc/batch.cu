@@ -237,9 +237,20 @@ int put(edus_batch* b, void* d, const std::vector<T>& h) {
 }
 
 // A table in the reference's layout to the instance's planes: sent as it lies and
-// laid out by the device, through the scratch (room for the widest table).
+// laid out by the device, through the scratch (room for the widest table); without
+// scratch the host lays it out.
 template <class T>
 int put_planes(edus_batch* b, const std::vector<cd>& src, int nk, int n, int comps, bool full, T* dst, double2* scratch) {
+  if (!scratch) {
+    const int ne = full ? n * n : n * (n + 1) / 2;
+    std::vector<T> pl((size_t)comps * ne * nk);
+    for (int k = 0; k < nk; k++)
+      for (int i = 0; i < n; i++)
+        for (int j = full ? 0 : i; j < n; j++)
+          for (int x = 0; x < comps; x++)
+            pl[((size_t)x * ne + (full ? i * n + j : tri_index(i, j, n))) * nk + k] = mkc<T>(src[(((size_t)k * n + i) * n + j) * comps + x]);
+    return put(b, (void*)dst, pl);
+  }
   BCK(cudaMemcpyAsync(scratch, src.data(), sizeof(cd) * src.size(), cudaMemcpyHostToDevice, b->stream));
   b->h2d_bytes += (long long)(sizeof(cd) * src.size());
   BCK(launch_to_planes(scratch, nk, n, comps, full, dst, b->stream));
@@ -252,7 +263,7 @@ int upload_model(edus_batch* b, const Problem& P, const Inst& I) {
   double2* scr = nullptr;
   if (cudaMallocAsync((void**)&scr, sizeof(double2) * 3 * n * n * nk, b->pool, b->stream) != cudaSuccess) {
     cudaGetLastError();
-    return fail(EDUS_ENOMEM, "batch: upload scratch of %zu bytes", sizeof(double2) * 3 * n * n * nk);
+    scr = nullptr;
   }
   int rc = put_planes(b, P.H, nk, n, 1, false, (T*)I.H, scr);
   if (!rc) rc = put_planes(b, P.D, nk, n, 3, false, (T*)I.D, scr);
@@ -266,7 +277,7 @@ int upload_model(edus_batch* b, const Problem& P, const Inst& I) {
   }
   // mixed precision: the state is the deviation from rho_eq
   if (!rc) rc = put_planes(b, P.P0, nk, n, 1, false, I.Peq ? const_cast<double2*>(I.Peq) : I.P0, scr);
-  cudaFreeAsync(scr, b->stream);
+  if (scr) cudaFreeAsync(scr, b->stream);
   return rc;
 }
 
@@ -762,17 +773,19 @@ int run_chunk(edus_batch* b, LaunchTimer* tm = nullptr) {
 // Device memory to the caller's (pageable) memory: two pinned buffers take turns,
 // the copy of one over PCIe running while the threads of the host empty the other.
 // The driver's own path for pageable memory fills the caller's fresh pages on one
-// thread. Waits for the stream.
+// thread; it takes small pieces, and all where pinned memory cannot be had. Waits for
+// the stream.
 cudaError_t copy_out(edus_batch* b, void* dst, const void* src, size_t bytes) {
-  if (bytes < kStageBytes / 4) {
+  bool staged = bytes >= kStageBytes / 4;
+  for (int q = 0; q < 2 && staged; q++) {
+    if (!b->stage[q] && cudaHostAlloc(&b->stage[q], kStageBytes, cudaHostAllocDefault) != cudaSuccess) b->stage[q] = nullptr;
+    if (!b->stage_ev[q] && cudaEventCreateWithFlags(&b->stage_ev[q], cudaEventDisableTiming) != cudaSuccess) b->stage_ev[q] = nullptr;
+    staged = b->stage[q] && b->stage_ev[q];
+    if (!staged) cudaGetLastError();
+  }
+  if (!staged) {
     cudaError_t e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, b->stream);
     return e == cudaSuccess ? cudaStreamSynchronize(b->stream) : e;
-  }
-  for (int q = 0; q < 2; q++) {
-    cudaError_t e = cudaSuccess;
-    if (!b->stage[q]) e = cudaHostAlloc(&b->stage[q], kStageBytes, cudaHostAllocDefault);
-    if (e == cudaSuccess && !b->stage_ev[q]) e = cudaEventCreateWithFlags(&b->stage_ev[q], cudaEventDisableTiming);
-    if (e != cudaSuccess) return e;
   }
   const size_t nchunk = (bytes + kStageBytes - 1) / kStageBytes;
   auto size = [&](size_t c) { return std::min(kStageBytes, bytes - c * kStageBytes); };
@@ -1245,14 +1258,31 @@ int edus_batch_get_state(edus_batch* b, int32_t slot, double* rho) {
   }
   BCK(cudaSetDevice(b->device));
   // full matrices on the device (mixed precision keeps the deviation from
-  // rho_eq), then out through the batch's pinned buffers
-  const size_t bytes = sizeof(double2) * (size_t)s->n * s->n * s->nk;
+  // rho_eq), then out through the batch's pinned buffers; the host lays out the
+  // planes where the device has no room for the matrices
+  const int n = s->n, nk = s->nk;
+  const size_t bytes = sizeof(double2) * (size_t)n * n * nk;
   double2* full = nullptr;
   if (cudaMallocAsync((void**)&full, bytes, b->pool, b->stream) != cudaSuccess) {
     cudaGetLastError();
-    return fail(EDUS_ENOMEM, "batch: %zu bytes for the state's matrices", bytes);
+    std::vector<double2> pl((size_t)s->ntri * nk), eq(s->inst.Peq ? pl.size() : 0);
+    BCK(cudaMemcpyAsync(pl.data(), s->inst.P0, sizeof(double2) * pl.size(), cudaMemcpyDeviceToHost, b->stream));
+    if (s->inst.Peq)
+      BCK(cudaMemcpyAsync(eq.data(), s->inst.Peq, sizeof(double2) * eq.size(), cudaMemcpyDeviceToHost, b->stream));
+    BCK(cudaStreamSynchronize(b->stream));
+    b->d2h_bytes += (long long)(sizeof(double2) * (pl.size() + eq.size()));
+    cd* o = (cd*)rho;
+    for (int k = 0; k < nk; k++)
+      for (int i = 0; i < n; i++)
+        for (int j = i; j < n; j++) {
+          const size_t q = (size_t)tri_index(i, j, n) * nk + k;
+          const double2 v = s->inst.Peq ? cadd(pl[q], eq[q]) : pl[q];
+          o[((size_t)k * n + i) * n + j] = cd(v.x, v.y);
+          if (i != j) o[((size_t)k * n + j) * n + i] = cd(v.x, -v.y);
+        }
+    return 0;
   }
-  cudaError_t e = launch_from_planes(s->inst.P0, s->inst.Peq, s->nk, s->n, full, b->stream);
+  cudaError_t e = launch_from_planes(s->inst.P0, s->inst.Peq, nk, n, full, b->stream);
   if (e == cudaSuccess) e = copy_out(b, rho, full, bytes);
   cudaFreeAsync(full, b->stream);
   BCK(e);

@@ -10,9 +10,9 @@
 #include <stdlib.h>
 #include <string.h>
 
-enum { O_SMS, O_COOP, O_CLUSTERS, O_BLOCKS, O_ENCODE, O_MALLOC_MAX, O_POOL_MAX, O_PINNED_MAX, N_OPT };
-static long opt[N_OPT] = {148, 1, 64, 1, 0, 1L << 40, 1L << 40, 1L << 40};
-static const char* opt_name[N_OPT] = {"sms", "cooperative", "max_clusters", "blocks_per_sm", "encode_result", "malloc_max", "pool_max", "pinned_max"};
+enum { O_SMS, O_COOP, O_CLUSTERS, O_BLOCKS, O_ENCODE, O_MALLOC_MAX, O_POOL_REFUSED, O_PINNED_MAX, N_OPT };
+static long opt[N_OPT] = {148, 1, 64, 1, 0, 1L << 40, -1, 1L << 40};
+static const char* opt_name[N_OPT] = {"sms", "cooperative", "max_clusters", "blocks_per_sm", "encode_result", "malloc_max", "pool_refused", "pinned_max"};
 
 int fake_set(const char* name, long v) {
   for (int i = 0; i < N_OPT; i++)
@@ -267,7 +267,7 @@ cudaError_t cudaMalloc(void** p, size_t n) { return take(p, n, opt[O_MALLOC_MAX]
 cudaError_t cudaFree(void* p) { return give(p); }
 cudaError_t cudaMallocFromPoolAsync(void** p, size_t n, cudaMemPool_t q, cudaStream_t s) {
   (void)q, (void)s;
-  return take(p, n, opt[O_POOL_MAX], 0);
+  return take(p, n, (long)n == opt[O_POOL_REFUSED] ? -1 : 1L << 40, 0);  /* a pool refuses this size */
 }
 cudaError_t cudaFreeAsync(void* p, cudaStream_t s) {
   (void)s;

@@ -1,5 +1,7 @@
 """Host paths over a stand-in CUDA runtime: calls that fail, work that shares a
 device, devices other than the current one. No GPU needed."""
+import pytest
+
 from host_paths import run_host
 
 
@@ -58,4 +60,34 @@ def test_whole_run_in_one_launch_only_where_nothing_else_is_at_work(workdir):
     batch.add(cou)
     batch.close()                            # released without being polled
     assert run(b) == (1, 0)
+    """)
+
+
+@pytest.mark.parametrize("precision", ["FP64", "MIXED"])
+def test_batch_without_layout_scratch(workdir, precision):
+    """Device memory that is short: tables and states are laid out on the host (mixed
+    precision keeps the state as a deviation from the ground state)."""
+    run_host(workdir, """
+    n, nk = 8, 100
+    pb = problem(W.wannier(d + "/a", nw=n, nside=3, n=10, t_fin_fs=0.1, name="W"))
+    limit("pool_refused", 48 * n * n * nk)      # scratch of the tables
+    b = E.Batch(precision=abi.EDUS_PREC_%s)
+    s = b.add(pb)
+    limit("pool_refused", 16 * n * n * nk)      # the state's matrices
+    got, P0 = b.get_state(s), pb.get("P0")
+    assert launches("k_to_planes") == launches("k_from_planes") == 0
+    assert np.array_equal(got, np.triu(P0) + np.conj(np.triu(P0, 1)).transpose(0, 2, 1))
+    """ % precision)
+
+
+def test_batch_state_without_pinned_buffers(workdir):
+    """No pinned memory: a large state comes out through pageable memory."""
+    run_host(workdir, """
+    pb = problem(W.hbn_rk4(d + "/a", n=90, t_fin_fs=0.1))  # 1.2 MB of matrices
+    b = E.Batch()
+    s = b.add(pb)
+    limit("pinned_max", 1024)
+    assert b.get_state(s).shape == (8100, 3, 3)
+    limit("pinned_max", 1 << 40)
+    assert b.get_state(s).shape == (8100, 3, 3)
     """)
