@@ -12,6 +12,7 @@
 #include <cmath>
 #include <cstring>
 #include <map>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -111,7 +112,8 @@ struct edus_batch {
   double device_ms = 0, kpoint_steps = 0;
   long long launches = 0;
   long long h2d_bytes = 0, d2h_bytes = 0;
-  // pinned buffers of copy_out, allocated by the first state that is read
+  // pinned buffers of copy_out, allocated by the first state that is read; one reader at a time
+  std::mutex stage_mu;
   void* stage[2] = {nullptr, nullptr};
   cudaEvent_t stage_ev[2] = {nullptr, nullptr};
 };
@@ -777,6 +779,8 @@ int run_chunk(edus_batch* b, LaunchTimer* tm = nullptr) {
 // the stream.
 cudaError_t copy_out(edus_batch* b, void* dst, const void* src, size_t bytes) {
   bool staged = bytes >= kStageBytes / 4;
+  std::unique_lock<std::mutex> lk(b->stage_mu, std::defer_lock);
+  if (staged) lk.lock();
   for (int q = 0; q < 2 && staged; q++) {
     if (!b->stage[q] && cudaHostAlloc(&b->stage[q], kStageBytes, cudaHostAllocDefault) != cudaSuccess) b->stage[q] = nullptr;
     if (!b->stage_ev[q] && cudaEventCreateWithFlags(&b->stage_ev[q], cudaEventDisableTiming) != cudaSuccess) b->stage_ev[q] = nullptr;

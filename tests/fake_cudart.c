@@ -267,7 +267,10 @@ cudaError_t cudaMalloc(void** p, size_t n) { return take(p, n, opt[O_MALLOC_MAX]
 cudaError_t cudaFree(void* p) { return give(p); }
 cudaError_t cudaMallocFromPoolAsync(void** p, size_t n, cudaMemPool_t q, cudaStream_t s) {
   (void)q, (void)s;
-  return take(p, n, (long)n == opt[O_POOL_REFUSED] ? -1 : 1L << 40, 0);  /* a pool refuses this size */
+  static unsigned char fresh = 0;
+  const cudaError_t e = take(p, n, (long)n == opt[O_POOL_REFUSED] ? -1 : 1L << 40, 0); /* this size is refused */
+  if (e == cudaSuccess) memset(*p, ++fresh, n); /* not cleared, and no two alike */
+  return e;
 }
 cudaError_t cudaFreeAsync(void* p, cudaStream_t s) {
   (void)s;

@@ -91,3 +91,26 @@ def test_batch_state_without_pinned_buffers(workdir):
     limit("pinned_max", 1 << 40)
     assert b.get_state(s).shape == (8100, 3, 3)
     """)
+
+
+def test_states_of_one_batch_read_by_two_threads(workdir):
+    """The pinned buffers serve one reader at a time. (Kernels do not run here: each
+    reader's matrices are what its own device buffer holds, one byte all over.)"""
+    run_host(workdir, """
+    import threading
+    pb = problem(W.hbn_rk4(d + "/a", n=90, t_fin_fs=0.1))  # 1.2 MB of matrices
+    b = E.Batch()
+    s, t = b.add(pb), b.add(pb)
+    got = {}
+    second = threading.Thread(target=lambda: got.update(second=b.get_state(t)))
+    @C.CFUNCTYPE(None)
+    def wait():  # the first reader's copy is on its way
+        F.fake_on_wait(None)
+        second.start()
+        second.join(0.5)
+    F.fake_on_wait(wait)
+    got["first"] = b.get_state(s)
+    second.join()
+    one, two = (set(got[q].view(np.uint8).ravel()) for q in ("first", "second"))
+    assert len(one) == len(two) == 1 and one != two
+    """)
