@@ -386,12 +386,11 @@ void detect_lattice(const Problem& P, Inst& I) {
 // Mixed precision: H(k), D(k) on the tensor cores (cuda/tc_contract.cu, split
 // TF32), band energies in FP64, then the eigensolve and dH/dk on the FP64 matrix
 // the dynamics uses.
-int build_model_tc(edus_batch* b, const Problem& P, const Inst& I) {
+int build_model_tc(edus_batch* b, const Problem& P, const Inst& I, TcForm form) {
   const int n = P.ncv, nt = n * (n + 1) / 2, nk = P.nk, nr = P.nrpts;
   // H and D on the tensor cores; dH/dk, an observable-only table whose k sums
   // cancel strongly, is the reference's stencil over an FP64 H(k) (CUDA cores)
   const int ncomp = 4;
-  const TcForm form = tc_gemm_form();
   const int kp = tc_depth(nr, form), ncols = 2 * ncomp * nt;
   const size_t csize = tc_c_size(nk, nt, form);
   // upper coefficients of H(R) and the symmetrised dipoles; the scale of a GEMM
@@ -462,6 +461,10 @@ int build_model_tc(edus_batch* b, const Problem& P, const Inst& I) {
   t.hdiagR = dh;
   t.op.A = (uint16_t*)carve(sizeof(uint16_t) * (size_t)nk * kp);
   t.op.C = (double*)carve(sizeof(double) * csize);
+  if (!tc_maps(t.op, nk, nt, nr)) {
+    cudaFreeAsync(base, b->stream);
+    return build_model_tc(b, P, I, TcForm::cpasync);
+  }
   t.H32 = (float2*)I.H;
   t.D32 = (float2*)I.D;
   t.Hdiag = (double*)I.Hdiag;
@@ -1133,7 +1136,7 @@ int edus_batch_add(edus_batch* b, const edus_problem* pb, int64_t tag, int32_t* 
   if (P.model_deferred) {
     // (the exact segment sums hold up to 1024-deep segments, 512 R vectors)
     const bool tc = cmix(b, n) && b->opt.tc_contraction && P.p.conduction_shift <= 1e-16 && tc_seg_k(P.nrpts) <= 1024;
-    if ((rc = tc ? build_model_tc(b, P, I) : build_model_on_device(b, P, I))) return undo(rc);
+    if ((rc = tc ? build_model_tc(b, P, I, tc_gemm_form()) : build_model_on_device(b, P, I))) return undo(rc);
   } else {
     rc = cmix(b, n) ? upload_model<float2>(b, P, I) : upload_model<double2>(b, P, I);
     if (rc) return undo(rc);

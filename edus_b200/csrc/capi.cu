@@ -1937,9 +1937,7 @@ int edus_create(const edus_problem* pb, const edus_options* opt, edus_ctx** out)
     if (c->vg_tc) {
       // power-of-two scale of each GEMM column from max_R |c(R)| (bounds |Re|, |Im| of
       // e^{2 pi i A.R} c(R) for every A): every sliced value lies in [-1/2, 1/2]
-      const batch::TcForm form = batch::tc_gemm_form();
-      const int ncols = 8 * nt, kpad = batch::tc_depth(nr, form);
-      const size_t csize = batch::tc_c_size(nk, nt, form);
+      const int ncols = 8 * nt;
       std::vector<double> cs(ncols);
       for (int ce = 0; ce < 4 * nt; ce++) {
         double amax = 0.;
@@ -1947,11 +1945,7 @@ int edus_create(const edus_problem* pb, const edus_options* opt, edus_ctx** out)
         cs[2 * ce] = cs[2 * ce + 1] = amax > 0. ? std::ldexp(1.0, std::ilogb(amax) + 2) : 1.0;
       }
       double* dcs = nullptr;
-      uint16_t *dA = nullptr, *dB = nullptr;
-      double* dC = nullptr;
-      if ((rc = dalloc(c, &dcs, (size_t)ncols)) || (rc = dalloc(c, &dA, (size_t)nk * kpad)) ||
-          (rc = dalloc(c, &dB, (size_t)ncols * kpad)) || (csize && (rc = dalloc(c, &dC, csize))))
-        return bail(rc);
+      if ((rc = dalloc(c, &dcs, (size_t)ncols))) return bail(rc);
       if (cudaMemcpyAsync(dcs, cs.data(), sizeof(double) * ncols, cudaMemcpyHostToDevice, c->stream) != cudaSuccess)
         return bail(fail(EDUS_ECUDA, "velocity gauge: upload"));
       batch::TcVgArgs& g = c->vgt;
@@ -1963,10 +1957,16 @@ int edus_create(const edus_problem* pb, const edus_options* opt, edus_ctx** out)
       g.Rvec = dR;
       g.coef = dcoef;
       g.colscale = dcs;
-      g.op.form = form;
-      g.op.A = dA;
-      g.op.B = dB;
-      g.op.C = dC;
+      for (batch::TcForm form = batch::tc_gemm_form();; form = batch::TcForm::cpasync) {
+        const int kpad = batch::tc_depth(nr, form);
+        const size_t csize = batch::tc_c_size(nk, nt, form);
+        g.op = batch::TcOperands();
+        g.op.form = form;
+        if ((rc = dalloc(c, &g.op.A, (size_t)nk * kpad)) || (rc = dalloc(c, &g.op.B, (size_t)ncols * kpad)) ||
+            (csize && (rc = dalloc(c, &g.op.C, csize))))
+          return bail(rc);
+        if (batch::tc_maps(g.op, nk, nt, nr)) break;
+      }
       g.H = dH;
       g.D = dD;
       g.err = c->d_err;

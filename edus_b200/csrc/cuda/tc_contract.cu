@@ -808,14 +808,12 @@ cudaError_t gemm_planes(const TcOperands& o, T* H, T* D, int nk, int n, int ntri
   return cudaGetLastError();
 }
 
-// phase slices of the grid, zero segment padding of the coefficient slices, tensor maps
-cudaError_t prepare(TcOperands& o, const double* kpt, const double* Rvec, int nk, int ntri, int nr, cudaStream_t s) {
+// phase slices of the grid, zero segment padding of the coefficient slices
+cudaError_t prepare(const TcOperands& o, const double* kpt, const double* Rvec, int nk, int ntri, int nr, cudaStream_t s) {
   const int kpad = tc_depth(nr, o.form), ncols = 8 * ntri;
   k_phase_split<<<nk, 256, 0, s>>>(kpt, Rvec, nk, nr, tc_seg_k(nr), kpad, o.A);
   cudaError_t e = cudaGetLastError();
   if (e == cudaSuccess) e = cudaMemsetAsync(o.B, 0, sizeof(uint16_t) * (size_t)ncols * kpad, s);
-  if (e == cudaSuccess && o.form != TcForm::cpasync) e = encode_operand(&o.mapA, o.A, nk, kpad, TM);
-  if (e == cudaSuccess && o.form != TcForm::cpasync) e = encode_operand(&o.mapB, o.B, ncols, kpad, o.form == TcForm::planes ? TN3 : TN2);
   return e;
 }
 
@@ -839,7 +837,14 @@ TcForm tc_gemm_form() {
   return TcForm::planes;
 }
 
-cudaError_t tc_contract(TcArgs& a, cudaStream_t s) {
+bool tc_maps(TcOperands& o, int nk, int ntri, int nr) {
+  if (o.form == TcForm::cpasync) return true;
+  const int kpad = tc_depth(nr, o.form);
+  return encode_operand(&o.mapA, o.A, nk, kpad, TM) == cudaSuccess &&
+         encode_operand(&o.mapB, o.B, 8 * ntri, kpad, o.form == TcForm::planes ? TN3 : TN2) == cudaSuccess;
+}
+
+cudaError_t tc_contract(const TcArgs& a, cudaStream_t s) {
   const double zero[3] = {0., 0., 0.};
   cudaError_t e = prepare(a.op, a.kpt, a.Rvec, a.nk, a.ntri, a.nr, s);
   if (e == cudaSuccess) e = cut_coefficients(a.op, a.coef, a.Rvec, a.colscale, zero, a.ntri, a.nr, s);
@@ -849,7 +854,7 @@ cudaError_t tc_contract(TcArgs& a, cudaStream_t s) {
   return cudaGetLastError();
 }
 
-cudaError_t tc_vg_prepare(TcVgArgs& a, cudaStream_t s) { return prepare(a.op, a.kpt, a.Rvec, a.nk, a.ntri, a.nr, s); }
+cudaError_t tc_vg_prepare(const TcVgArgs& a, cudaStream_t s) { return prepare(a.op, a.kpt, a.Rvec, a.nk, a.ntri, a.nr, s); }
 
 cudaError_t tc_vg_stage(const TcVgArgs& a, cudaStream_t s) {
   cudaError_t e = cut_coefficients(a.op, a.coef, a.Rvec, a.colscale, a.A, a.ntri, a.nr, s);

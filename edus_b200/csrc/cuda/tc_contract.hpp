@@ -79,7 +79,10 @@ __host__ __device__ inline uint16_t tc_bf16(double v) {
   memcpy(&u, &f, 4);
   return (uint16_t)(u >> 16);
 }
-cudaError_t tc_contract(TcArgs& a, cudaStream_t s);
+// Tensor maps of A and B. False where the driver has none for these operands: the
+// caller then lays them out for `cpasync`, which needs no maps.
+bool tc_maps(TcOperands& o, int nk, int ntri, int nr);
+cudaError_t tc_contract(const TcArgs& a, cudaStream_t s);
 
 // Velocity gauge on the tensor cores: H(k + A), D(k + A) of every k point for
 // every RK4 stage as the exact-slice GEMM above. The phase slices of the grid
@@ -99,7 +102,7 @@ struct TcVgArgs {
   double2* D = nullptr;              // out [3][ntri][nk]
   int* err = nullptr;                // device error word (bounded waits)
 };
-cudaError_t tc_vg_prepare(TcVgArgs& a, cudaStream_t s);
+cudaError_t tc_vg_prepare(const TcVgArgs& a, cudaStream_t s);
 cudaError_t tc_vg_stage(const TcVgArgs& a, cudaStream_t s);
 
 }  // namespace batch

@@ -114,3 +114,24 @@ def test_states_of_one_batch_read_by_two_threads(workdir):
     one, two = (set(got[q].view(np.uint8).ravel()) for q in ("first", "second"))
     assert len(one) == len(two) == 1 and one != two
     """)
+
+
+def test_tensor_core_sums_without_tensor_maps(workdir):
+    """A driver that refuses the tensor maps: the sums run in the form that needs none."""
+    run_host(workdir, """
+    limit("encode_result", 1)
+    path = W.wannier(d + "/v", nw=8, nside=3, n=8, t_fin_fs=0.1, name="W")
+    text = open(path).read().replace("tdse{\\nWannier\\n", "tdse{\\nWannier\\nvelocity_gauge\\n")
+    open(path, "w").write(text)
+    c = E.Context(problem(path), precision=abi.EDUS_PREC_MIXED)
+    assert launches("k_tc_gemmE") == 1 and launches("k_scatter64") == 1
+    c.step(1)
+    b = E.Batch(precision=abi.EDUS_PREC_MIXED)
+    F.fake_clear()
+    b.add(problem(W.wannier(d + "/b", nw=8, nside=3, n=8, t_fin_fs=0.1, name="W"), defer_model=True))
+    assert launches("k_tc_gemmE") == 1 and launches("k_tc_planes") == 0 and launches("k_tc_gemm_tma") == 0
+    limit("encode_result", 0)
+    F.fake_clear()
+    b.add(problem(W.wannier(d + "/b", nw=8, nside=3, n=8, t_fin_fs=0.1, name="W"), defer_model=True))
+    assert launches("k_tc_planes") == 1 and launches("k_tc_gemmE") == 0
+    """)
