@@ -711,7 +711,7 @@ int dyn_enqueue_chunk(edus_ctx* c, int K, bool every) {
       memset(&rec, 0, sizeof(rec));
       CK(launch_observables(c->tb, c->d_cst, c->d_P0, c->coul ? c->d_hr : nullptr, c->coul, c->d_uev, c->P.p.current, c->P.p.tabs, c->d_part,
                             c->d_done, scaleJ, scaleTA, rec, c->d_log, c->d_ncond, c->d_pcmax, c->stream, d));
-      c->launches++;
+      c->launches += c->coul && c->d_uev ? 2 : 1;
       if (c->snap_on && c->d_snap) {
         CK(launch_snapshot(c->tb, c->d_P0, c->snap_ic, c->snap_jc, c->d_snap, c->stream, d));
         c->launches++;

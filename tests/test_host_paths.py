@@ -135,3 +135,50 @@ def test_tensor_core_sums_without_tensor_maps(workdir):
     b.add(problem(W.wannier(d + "/b", nw=8, nside=3, n=8, t_fin_fs=0.1, name="W"), defer_model=True))
     assert launches("k_tc_planes") == 1 and launches("k_tc_gemmE") == 0
     """)
+
+
+LAUNCH_COUNT = """
+    def coulomb8(kind):
+        # an 8-band Wannier model with small mean-field tables of two modes
+        w, n, nc = d + "/" + kind, 8, 2
+        path = W.wannier(w, nw=n, nside=3, n=8, t_fin_fs=0.2, it_res=2, name="W")
+        os.makedirs(w + "/Output/Coulomb")
+        for q in "ABCD":
+            with open(f"{w}/Output/Coulomb/{q}_coefft.txt", "w") as f:
+                f.write("1e-3 0 " * (nc * nc * n * n))
+        with open(w + "/Output/Coulomb/Screen_const_t.txt", "w") as f:
+            f.write("1e-3 0 " * (n * n))
+        with open(w + "/Output/Coulomb/V_Hartree_t.txt", "w") as f:
+            f.write("1e-3 " * (n * n))
+        text = open(path).read()
+        if kind == "adaptive":
+            text = text.replace("tdse{\\n", "tdse{\\ndynamical_dt_evolution\\nepsStepAbs 0.001\\n")
+        text += "\\nCoulomb{\\nqTF 0.01\\nNcut 2\\nepsilon_static 1.0\\nRytova_Keldysh\\nRead_Coulomb_from_files\\nlabelInput t\\n}\\n"
+        open(path, "w").write(text)
+        return path
+
+    def vgauge():
+        path = W.wannier(d + "/v", nw=8, nside=3, n=8, t_fin_fs=0.2, it_res=2, name="W")
+        text = open(path).read().replace("tdse{\\nWannier\\n", "tdse{\\nWannier\\nvelocity_gauge\\n")
+        open(path, "w").write(text)
+        return path
+
+    def adaptive3():
+        return W.hbn_rk4(d + "/d", n=8, t_fin_fs=0.2, it_res=2, solver="dynamical_dt_evolution\\nepsStepAbs 0.001\\n")
+
+    kind = "%s"
+    path = dict(hbn=lambda: W.hbn_rk4(d + "/h", n=8, t_fin_fs=0.2, it_res=2), coulomb8=lambda: coulomb8("constant"),
+                vgauge=vgauge, adaptive8=lambda: coulomb8("adaptive"), adaptive3=adaptive3)[kind]()
+    prec = abi.EDUS_PREC_MIXED if kind == "vgauge" else abi.EDUS_PREC_FP64
+    c = E.Context(problem(path), use_graphs=False, precision=prec)
+    end = C.CFUNCTYPE(None)(F.fake_clear_flag)  # an adaptive run ends with the chunk that is waited for
+    F.fake_on_wait(end)
+    F.fake_clear()
+    c.run()
+    assert launches() > 0 and c.last_timing()[1] == launches()
+"""
+
+
+@pytest.mark.parametrize("kind", ["hbn", "coulomb8", "vgauge", "adaptive3", "adaptive8"])
+def test_launch_count_is_the_number_of_launches(workdir, kind):
+    run_host(workdir, LAUNCH_COUNT % kind)
