@@ -973,7 +973,7 @@ int loop_prepare(edus_ctx* c) {
   a.ncomp = 0;
   for (int x = 0; x < 3; x++)
     if (((pmask | qmask) >> x) & 1) a.comp[a.ncomp++] = x;
-  const LoopPlan p = loop_plan(c->tb, a.nb_sel, a.ngc, a.ncomp, sms);
+  const LoopPlan p = loop_plan(c->tb, a.nb_sel, a.ngc, a.ncomp, sms, ab);
   if (p.blocks == 0) return 0;
   a.stride = sizeof(LoopStep) + sizeof(double) * a.ngc;
   std::vector<unsigned char> tab(a.stride * nsteps, 0);

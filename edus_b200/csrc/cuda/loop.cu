@@ -614,29 +614,53 @@ __global__ void __launch_bounds__(MAXT) k_loop(const __grid_constant__ LoopArgs 
   }
 }
 
+// Launch attributes of a plan, for the launch and for the question whether it fits.
+template <int N, bool AB, int MAXT, bool CL>
+struct LoopLaunch {
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute at[1];
+  cudaError_t prepare(const LoopPlan& p, cudaStream_t s) {
+    cudaError_t e = cudaFuncSetAttribute(k_loop<N, AB, MAXT, CL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem);
+    if (e == cudaSuccess && CL && p.blocks + 1 > 8)
+      e = cudaFuncSetAttribute(k_loop<N, AB, MAXT, CL>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    cfg.gridDim = dim3(p.blocks + 1);
+    cfg.blockDim = dim3(p.threads);
+    cfg.dynamicSmemBytes = p.smem;
+    cfg.stream = s;
+    if (CL) {
+      at[0].id = cudaLaunchAttributeClusterDimension;
+      at[0].val.clusterDim.x = p.blocks + 1;
+      at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    } else {
+      at[0].id = cudaLaunchAttributeCooperative;
+      at[0].val.cooperative = 1;
+    }
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return e;
+  }
+};
+
 template <int N, bool AB, int MAXT, bool CL>
 cudaError_t loop_launch_t(const LoopArgs& a, const LoopPlan& p, cudaStream_t s) {
-  cudaError_t e = cudaFuncSetAttribute(k_loop<N, AB, MAXT, CL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem);
-  if (e == cudaSuccess && CL && p.blocks + 1 > 8)
-    e = cudaFuncSetAttribute(k_loop<N, AB, MAXT, CL>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-  if (e != cudaSuccess) return e;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(p.blocks + 1);
-  cfg.blockDim = dim3(p.threads);
-  cfg.dynamicSmemBytes = p.smem;
-  cfg.stream = s;
-  cudaLaunchAttribute at[1];
-  if (CL) {
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = p.blocks + 1;
-    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
-  } else {
-    at[0].id = cudaLaunchAttributeCooperative;
-    at[0].val.cooperative = 1;
+  LoopLaunch<N, AB, MAXT, CL> l;
+  const cudaError_t e = l.prepare(p, s);
+  return e == cudaSuccess ? cudaLaunchKernelEx(&l.cfg, k_loop<N, AB, MAXT, CL>, a) : e;
+}
+
+// All blocks of the plan resident at once.
+template <int N, bool AB, int MAXT, bool CL>
+bool loop_fits_t(const LoopPlan& p, int sms) {
+  LoopLaunch<N, AB, MAXT, CL> l;
+  int n = 0;
+  cudaError_t e = l.prepare(p, nullptr);
+  if (e == cudaSuccess && CL) e = cudaOccupancyMaxActiveClusters(&n, k_loop<N, AB, MAXT, CL>, &l.cfg);
+  if (e == cudaSuccess && !CL) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_loop<N, AB, MAXT, CL>, p.threads, p.smem);
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    return false;
   }
-  cfg.attrs = at;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, k_loop<N, AB, MAXT, CL>, a);
+  return CL ? n >= 1 : (long long)n * sms >= p.blocks + 1;
 }
 
 template <int N, bool AB>
@@ -645,13 +669,27 @@ cudaError_t loop_launch(const LoopArgs& a, const LoopPlan& p, cudaStream_t s) {
   return p.small ? loop_launch_t<N, AB, kLoopSmall, false>(a, p, s) : loop_launch_t<N, AB, kLoopThreads, false>(a, p, s);
 }
 
+template <int N, bool AB>
+bool loop_fits(const LoopPlan& p, int sms) {
+  if (p.cluster) return p.small && loop_fits_t<N, AB, kLoopSmall, true>(p, sms);
+  return p.small ? loop_fits_t<N, AB, kLoopSmall, false>(p, sms) : loop_fits_t<N, AB, kLoopThreads, false>(p, sms);
+}
+
 template <int N>
 size_t loop_smem(const DevTables& tb, bool small, int nb, int ngc, int ncomp, bool cluster) {
   return small ? LoopSmem<N, kLoopSmall>(nullptr, tb, nb, ngc, ncomp, cluster).bytes
                : LoopSmem<N, kLoopThreads>(nullptr, tb, nb, ngc, ncomp, cluster).bytes;
 }
 
-}  // namespace
+bool loop_plan_fits(int n, bool ab, const LoopPlan& p, int sms) {
+#define X(n) \
+  case n: return ab ? loop_fits<n, true>(p, sms) : loop_fits<n, false>(p, sms);
+  switch (n) {
+    X(1) X(2) X(3) X(4) X(5)
+    default: return false;
+  }
+#undef X
+}
 
 // One block per SM, one of them adding up the instants; a block of at least 128
 // threads (with fewer a block, more blocks only lengthen the barrier) and at most
@@ -659,13 +697,13 @@ size_t loop_smem(const DevTables& tb, bool small, int nb, int ngc, int ncomp, bo
 // of up to 16 with the hardware barrier. Larger grids, the mean field (whose
 // transforms are bound by shared memory, 24.4 us a step here against 22.2 with
 // the launch per stage on 120 x 120) and 8 and 16 bands keep the launch per stage.
-LoopPlan loop_plan(const DevTables& tb, int nb, int ngc, int ncomp, int sms) {
+LoopPlan loop_shape(const DevTables& tb, int nb, int ngc, int ncomp, int sms, bool cluster) {
   LoopPlan p;
-  if (tb.n < 1 || tb.n > 5 || tb.h) return p;
+  if (tb.n < 1 || tb.n > 5 || tb.h || sms < 2) return p;
   const int nt = tb.ntri;
   const int kt_min = (128 + nt - 1) / nt;
   int blocks = std::min((tb.nk + kt_min - 1) / kt_min, sms - 1);
-  p.cluster = (tb.nk + 14) / 15 <= kLoopSmall / nt;
+  p.cluster = cluster && (tb.nk + 14) / 15 <= kLoopSmall / nt;
   if (p.cluster) blocks = std::min(blocks, 15);
   p.kt = (tb.nk + blocks - 1) / blocks;
   blocks = (tb.nk + p.kt - 1) / p.kt;
@@ -683,6 +721,17 @@ LoopPlan loop_plan(const DevTables& tb, int nb, int ngc, int ncomp, int sms) {
   p.threads = threads;
   p.part = (size_t)2 * 32 * blocks;
   p.blocks = blocks;
+  return p;
+}
+
+}  // namespace
+
+// The first form whose blocks the device holds at once: it may not place so wide a
+// cluster, or lend the process fewer SMs than it has.
+LoopPlan loop_plan(const DevTables& tb, int nb, int ngc, int ncomp, int sms, bool ab) {
+  LoopPlan p = loop_shape(tb, nb, ngc, ncomp, sms, true);
+  if (p.blocks > 0 && p.cluster && !loop_plan_fits(tb.n, ab, p, sms)) p = loop_shape(tb, nb, ngc, ncomp, sms, false);
+  if (p.blocks > 0 && !loop_plan_fits(tb.n, ab, p, sms)) p = LoopPlan();
   return p;
 }
 

@@ -53,7 +53,7 @@ struct LoopPlan {
   size_t smem = 0;
   size_t part = 0;  // scratch doubles
 };
-LoopPlan loop_plan(const DevTables& tb, int nb, int ngc, int ncomp, int sms);
+LoopPlan loop_plan(const DevTables& tb, int nb, int ngc, int ncomp, int sms, bool ab);
 cudaError_t launch_loop(const LoopArgs& a, const LoopPlan& p, cudaStream_t s);
 
 }  // namespace edus

@@ -182,3 +182,27 @@ LAUNCH_COUNT = """
 @pytest.mark.parametrize("kind", ["hbn", "coulomb8", "vgauge", "adaptive3", "adaptive8"])
 def test_launch_count_is_the_number_of_launches(workdir, kind):
     run_host(workdir, LAUNCH_COUNT % kind)
+
+
+@pytest.mark.parametrize("solver", ["", "Adams_Bashforth 4\\n"])
+def test_whole_run_where_its_blocks_cannot_be_resident(workdir, solver):
+    """A device that does not place a cluster of 16 blocks, or not all blocks at once: the
+    cooperative grid instead of the cluster, and the launch per stage instead of both."""
+    run_host(workdir, """
+    def run(n):
+        c = E.Context(problem(W.hbn_rk4(d + "/a", n=n, t_fin_fs=0.1, solver="%s")))
+        F.fake_clear()
+        c.run()
+        assert c.clock()[0] > 0
+        return launches("Li384ELb1E"), launches("Li384ELb0E"), launches("k_rhs_ep") > 0
+    assert run(24) == (1, 0, False)     # one cluster
+    assert run(60) == (0, 1, False)
+    limit("max_clusters", 0)
+    assert run(24) == (0, 1, False)
+    limit("blocks_per_sm", 0)
+    assert run(24) == (0, 0, True) and run(60) == (0, 0, True)
+    limit("blocks_per_sm", 1)
+    limit("max_clusters", 8)
+    limit("sms", 1)                     # nothing left to step on beside the block that adds up
+    assert run(24) == (0, 0, True)
+    """ % solver)
