@@ -61,3 +61,22 @@ def test_adaptive_run_matches_the_host_loop(workdir, model, n, monkeypatch):
     b.run()
     assert a.clock()[0] == b.clock()[0]
     assert np.abs(a.get_state() - b.get_state()).max() < 1e-10  # the step size carries the rounding of a small change
+
+
+# the terms that are left out are zero for finite states only: 0 x inf is not
+@pytest.mark.parametrize("model,n", [("Vampa2015", 10), (HBN, 6), (8, 6)])
+@pytest.mark.parametrize("value", [np.inf, -np.inf, np.nan, 1e300])
+def test_state_that_is_not_finite_reaches_every_neighbour(workdir, model, n, value):
+    p = E.parse_input(write(workdir, model, n))
+    pb = E.Problem(p, workdir)
+    ctx, o = E.Context(pb), Oracle(p, workdir)
+    P = pb.get("P0")
+    P[n + 1, 0, 1] = complex(0.0, value)
+    P[n + 1, 1, 0] = complex(0.0, -value)
+    EF = [0.0, 0.0, 4e-4, 0.0, 0.0, 0.0]
+    ctx.slot_set(abi.SLOT_P0, P)
+    ctx.get_derivative(abi.SLOT_P0, EF, p.probe.wl, 1)
+    g, r = ctx.slot_get(abi.SLOT_PV), o.rhs(P, EF, p.probe.wl, 1)
+    upper = np.triu(np.ones(P.shape[1:], bool))
+    assert np.array_equal(np.isfinite(g)[:, upper], np.isfinite(r)[:, upper])
+    assert np.isfinite(value) == np.isfinite(g).all()
