@@ -1260,6 +1260,10 @@ int edus_batch_get_state(edus_batch* b, int32_t slot, double* rho) {
   if (!s || !rho || s->status == EDUS_INST_FREE) return fail(EDUS_EINVAL, "bad slot");
   if (s->sub) {
     int rc = edus_get_state(s->sub, rho);
+    // (the first read takes room for the matrices)
+    const int64_t bytes = (int64_t)ctx_device_bytes(s->sub);
+    b->bytes_used += bytes - s->bytes;
+    s->bytes = bytes;
     if (!rc) b->d2h_bytes += (long long)(16 * (size_t)s->nk * s->n * s->n);
     return rc;
   }

@@ -1271,9 +1271,9 @@ size_t ctx_device_bytes(const edus_ctx* c) { return c ? c->dev_bytes : 0; }
 
 double ctx_last_ms(const edus_ctx* c) { return c ? c->last_ms : 0.0; }
 
-// Upper bound of the device memory edus_create takes for a problem: the
+// Upper bound of the device memory a context takes for a problem: the
 // state, table and ring planes, the observable log, the Coulomb scratch and
-// the snapshot slots, with a margin.
+// the snapshot slots, with a margin that holds the matrices of a state that is read.
 int64_t ctx_footprint_estimate(const Problem& P) {
   const double n = P.ncv, nk = P.nk, nt = n * (n + 1) / 2, plane = 16.0 * nt * nk;
   const int order = P.p.solver == EDUS_SOLVER_RK4 ? 0 : P.p.order;

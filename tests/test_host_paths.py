@@ -206,3 +206,19 @@ def test_whole_run_where_its_blocks_cannot_be_resident(workdir, solver):
     limit("sms", 1)                     # nothing left to step on beside the block that adds up
     assert run(24) == (0, 0, True)
     """ % solver)
+
+
+def test_batch_accounts_for_the_memory_a_mean_field_state_is_read_through(workdir):
+    run_host(workdir, """
+    pb = problem(W.hbn_coulomb(d + "/a", n=24, t_fin_fs=0.1))
+    b = E.Batch()
+    before = F.fake_held()
+    s = b.add(pb)
+    b.advance(16)
+    b.get_state(s)
+    used = b.stats()["bytes_used"]
+    assert used == F.fake_held() - before <= b.footprint(pb)
+    b.release(s)
+    used = b.stats()["bytes_used"]
+    assert used == 0 and F.fake_held() == before
+    """)
