@@ -11,6 +11,7 @@ import pytest
 import edus_b200 as E
 from edus_b200 import abi
 from edus_b200 import workloads as W
+from conftest import GOLDEN_INPUT
 
 pytestmark = pytest.mark.gpu
 
@@ -36,6 +37,9 @@ AB4 = "Adams_Bashforth 4\nAdams_Bashforth_RK4_startup\n"
     ("hbn", 30, 34, "", True),     # the first grid past it
     ("hbn", 60, 62, AB4, True),    # last block partly filled
     ("hbn", 98, 98, "", True),     # more than kLoopSmall threads a block
+    ("hbn", 98, 98, AB4, True),
+    ("hbn", 118, 122, AB4, True),
+    (5, 66, 66, AB4, True),
     ("hbn", 124, 124, "", True),   # 105 k points a block, the last that fits
     ("hbn", 126, 126, "", False),  # launch per stage
     (2, 12, 14, "", True),
@@ -68,6 +72,41 @@ def test_one_launch_matches_launch_per_stage(workdir, kind, n1, n2, solver, one)
 @pytest.mark.parametrize("kind,n1,n2,solver", [("hbn", 4, 4, AB4), ("hbn", 6, 6, ""), ("hbn", 18, 22, AB4), ("hbn", 30, 32, AB4), (2, 24, 26, ""), (5, 18, 20, AB4)])
 def test_one_cluster_matches_launch_per_stage(workdir, kind, n1, n2, solver):
     test_one_launch_matches_launch_per_stage(workdir, kind, n1, n2, solver, True)
+
+
+def compare(pb):
+    """One launch against the launch per stage: state, every field of the records."""
+    a, b = E.Context(pb), E.Context(pb, use_graphs=False)
+    a.run()
+    assert a.last_timing()[1] == 1
+    b.run()
+    assert np.abs(a.get_state() - b.get_state()).max() <= 1e-13
+    la, lb = a.obs(), b.obs()
+    assert len(la) == len(lb) > 2
+    for q in la[0]:
+        x, y = np.array([o[q] for o in la]), np.array([o[q] for o in lb])
+        assert np.abs(x - y).max() <= 1e-12, q
+    return lb
+
+
+# a decaying core hole (relaxation), circular pump, probe on the core, transient absorption:
+# one cluster, many blocks, blocks of more than kLoopSmall threads
+@pytest.mark.parametrize("n1,n2", [(12, 14), (40, 40), (100, 100)])
+@pytest.mark.parametrize("solver", ["Adams_Bashforth 5", ""])
+def test_core_hole_in_one_launch(workdir, n1, n2, solver):
+    text = open(GOLDEN_INPUT).read().replace("1 70 70", f"1 {n1} {n2}").replace("Adams_Bashforth\n", solver + "\n")
+    text = "\n".join(x for x in text.splitlines() if not x.startswith("PrintPopulation")) + "\n"
+    text = text.replace("t_fin 1650.36549334624544 au", "t_fin 92.0 au")  # the probe follows the pump
+    with open(workdir + "/input.txt", "w") as f:
+        f.write(text)
+    log = compare(E.Problem(E.parse_input(workdir + "/input.txt"), workdir))
+    assert max(np.abs(o["tabs"]).max() for o in log) > 0 and max(np.abs(o["EF_probe"]).max() for o in log) > 0
+
+
+# Hermitian dipoles, whose lower elements are the conjugates
+@pytest.mark.parametrize("nb,n", [((1, 1), 12), ((1, 2), 40)])
+def test_crystal_model_in_one_launch(workdir, nb, n):
+    compare(E.Problem(E.parse_input(W.crystal(workdir, nb=nb, nkf=13, n=n, duration=2.0, t_fin_fs=0.6)), workdir))
 
 
 def test_run_of_several_launches_keeps_the_history(workdir):
