@@ -320,7 +320,7 @@ int run_coulomb(edus_ctx* c, const double2* src) {
   return prof_mark(c, 1, false);
 }
 
-// The terms of a stage that are not exact zeros. A shell weight below 1e-12 of
+// The terms of a stage that count. A shell weight below 1e-12 of
 // the largest is least-squares noise of the weight fit (1e-21 against 1e3 for the
 // diagonal shell of a square grid), its terms far below the FP64 resolution of the
 // sum; batches leave the same ones out. With a state or dipoles that are not

@@ -18,8 +18,9 @@
 //   70 x 70 with core-hole decay, AB5: 5.5 us a step, 10.5 before
 //
 // The blocks wait on one another, so the launch is cooperative (all blocks
-// resident) or one cluster; a wait is bounded and records kErrTimeout. Data
-// written by other blocks is read past L1.
+// resident) or one cluster. A wait on the cooperative grid is bounded and records
+// kErrTimeout; the cluster's hardware barrier has no bound: its blocks are placed
+// together and make the same barrier calls. Data written by other blocks is read past L1.
 //
 // Arithmetic: every element goes through the expressions of k_rhs_ep in the same
 // order, but for relaxation, whose products are formed once per k point.
@@ -50,7 +51,8 @@ struct TriL {
   }
 };
 
-// Most threads of a block: 168 registers each, or 96 for the largest grids.
+// Most threads of a block: 168 registers each, or 96 for the largest grids, which spill
+// (3 bands 340 bytes, 5 bands 400).
 constexpr int kLoopSmall = 384, kLoopThreads = 640;
 constexpr int kSumF = 3 * kPerX;   // current fields of a block partial
 

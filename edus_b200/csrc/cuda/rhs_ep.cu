@@ -12,10 +12,12 @@
 // thread per k this gives NT times the parallelism for the small grids of the
 // reference's workloads, where one solve has only 10^3-10^4 k points.
 //
-// Bound by L2: with 8 and 16 bands most of a stage's bytes are the stencil
+// Bound by latency: 96 x 96 with 8 bands has L2 at 19 %, L1 and shared memory at 66 %
+// and a third of the issue slots in use; most of a stage's loads are the stencil
 // gathers and the dipole planes. Stencil vectors orthogonal to the field (8 of 12
-// on a square grid with the field along an axis) and dipole components without a
-// field are left out: their terms are exact zeros. 96 x 96, 8 bands: 20.5 us a
+// on a square grid with the field along an axis), those whose shell weight is rounding
+// residue, and dipole components without a field are left out: their terms are zeros
+// or below the resolution of the sum. 96 x 96, 8 bands: 20.5 us a
 // stage, 25.2 with all of them; 30 x 34, 16 bands: 16.6, 17.6.
 //
 // 8 and 16 bands exchange full matrices (RowsEP): every operand of the commutator is
