@@ -153,6 +153,7 @@ struct edus_ctx {
   // initial state and dipoles finite, and the largest stencil weight (select_terms)
   bool finite = true;
   double wb_max = 0;
+  static constexpr double kNoWeight = 1e-16;
   double2* d_full = nullptr;  // matrices of state_from_dev, allocated on its first call
   double2* d_Pinit = nullptr;
   double2 *P0_start = nullptr, *Pa_start = nullptr;
@@ -320,11 +321,11 @@ int run_coulomb(edus_ctx* c, const double2* src) {
   return prof_mark(c, 1, false);
 }
 
-// The terms of a stage that count. A shell weight below 1e-12 of
-// the largest is least-squares noise of the weight fit (1e-21 against 1e3 for the
-// diagonal shell of a square grid), its terms far below the FP64 resolution of the
-// sum; batches leave the same ones out. With a state or dipoles that are not
-// finite 0 x NaN counts, and nothing is left out.
+// The terms of a stage that count. A shell weight below 1e-16 of the largest is
+// rounding residue of the least-squares fit (1e-24 to 1e-19 for the diagonal shell of a
+// square grid, 1.3e-16 at most on rectangular ones up to 126 k points a side): its terms are below the
+// FP64 resolution of the sum. With a state or dipoles that are not finite 0 x NaN
+// counts, and nothing is left out.
 void select_terms(const edus_ctx* c, StageArgs& a) {
   int pmask = 0, qmask = 0;
   if (a.dyn) {
@@ -345,7 +346,7 @@ void select_terms(const edus_ctx* c, StageArgs& a) {
   a.nsel = 0;
   for (int b = 0; b < c->tb.nnb; b++) {
     bool on = !c->finite;
-    if (std::fabs(c->hc.wb[b]) > 1e-12 * c->wb_max)
+    if (std::fabs(c->hc.wb[b]) > edus_ctx::kNoWeight * c->wb_max)
       for (int x = 0; x < 3; x++) on = on || (((pmask >> x) & 1) && c->hc.bvec[b][x] != 0.);
     if (on) a.sel[a.nsel++] = (unsigned char)b;
   }
@@ -976,7 +977,7 @@ int loop_prepare(edus_ctx* c) {
     if ((pmask >> x) & 1) comp[a.npc++] = x;
   for (int b = 0; b < P.nnb; b++) {
     bool on = !finite;
-    for (int q = 0; q < a.npc; q++) on = on || (c->hc.bvec[b][comp[q]] != 0. && std::fabs(c->hc.wb[b]) > 1e-12 * c->wb_max);
+    for (int q = 0; q < a.npc; q++) on = on || (c->hc.bvec[b][comp[q]] != 0. && std::fabs(c->hc.wb[b]) > edus_ctx::kNoWeight * c->wb_max);
     if (on) a.bsel[a.nb_sel++] = b;
   }
   a.nbp = std::max(12, (a.nb_sel + 5) / 6 * 6);
