@@ -690,7 +690,7 @@ int record_chunk(edus_batch* b, LaunchTimer* tm = nullptr) {
       ClassTab& c = kv.second;
       View v{b->d_insts, {b->d_it[0], b->d_it[1]}, c.d_tiles, c.d_ntiles, c.d_cinst, c.d_ntiles + 1};
       if (tm) BCK(tm->begin(c.n, 0, b->stream));
-      BCK(launch_obs(c.n, c.kt, cmix(b, c.n), v, parity, (int)b->slots.size(), c.ogrid, b->stream));
+      BCK(launch_obs(c.n, cmix(b, c.n), v, parity, (int)b->slots.size(), c.ogrid, b->stream));
       if (tm) BCK(tm->end(b->stream));
     }
     for (int st = 0; st < 4; st++)

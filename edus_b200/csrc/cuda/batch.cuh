@@ -100,7 +100,7 @@ cudaError_t launch_stage(int N, int kt, int occ, bool mixed, const View& v, int 
 // Observables of the instances due at this tick (it % res == 0) and the
 // step-counter advance of every instance of the class (batch_obs.cu);
 // max_inst bounds the class's instance table.
-cudaError_t launch_obs(int N, int kt, bool mixed, const View& v, int parity, int max_inst, int grid, cudaStream_t s);
+cudaError_t launch_obs(int N, bool mixed, const View& v, int parity, int max_inst, int grid, cudaStream_t s);
 // Persistent grid sizes (SMs x resident blocks) of the two kernels.
 int stage_grid(int N, int kt, int occ, bool mixed);
 int obs_grid(int N, bool mixed, int max_inst);

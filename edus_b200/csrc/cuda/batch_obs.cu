@@ -555,8 +555,7 @@ struct ObsForm<16, MIX> {
 };
 
 template <int N, bool MIX>
-cudaError_t obs_n(const View& v, int parity, int kt, int max_inst, int grid, cudaStream_t s) {
-  (void)kt;
+cudaError_t obs_n(const View& v, int parity, int max_inst, int grid, cudaStream_t s) {
   ObsForm<N, MIX>::kernel<<<grid, ObsForm<N, MIX>::NTHR, (size_t)(max_inst + 1) * sizeof(int), s>>>(v, parity);
   return cudaGetLastError();
 }
@@ -575,10 +574,10 @@ int obs_grid_n(int max_inst) {
 
 }  // namespace
 
-cudaError_t launch_obs(int N, int kt, bool mixed, const View& v, int parity, int max_inst, int grid, cudaStream_t s) {
+cudaError_t launch_obs(int N, bool mixed, const View& v, int parity, int max_inst, int grid, cudaStream_t s) {
   switch (N) {
 #define X(n) \
-  case n: return mixed ? obs_n<n, true>(v, parity, kt, max_inst, grid, s) : obs_n<n, false>(v, parity, kt, max_inst, grid, s);
+  case n: return mixed ? obs_n<n, true>(v, parity, max_inst, grid, s) : obs_n<n, false>(v, parity, max_inst, grid, s);
     X(2) X(3) X(4) X(5) X(8) X(16)
 #undef X
     default: return cudaErrorInvalidValue;
